@@ -288,3 +288,27 @@ def tolerance(case):
     if kind == "dflash":
         return {"rel": 3e-7, "max": 8e-7}       # path probabilities from such sums
     return "exact"
+
+
+def exact(case, seed):
+    """The computed numbers of `run` in 64 bits (log-sum-exps and what follows from them); the rest
+    of the outputs are ids, counts and flags, or (mixed, dflash) depend on which ids were chosen."""
+    kind = case["kind"]
+    if kind not in ("confidence", "logprobs"):
+        return None
+    x, *rest = prepare(case, seed)["args"]
+    top = torch.empty(x.shape[0], dtype=torch.float64, device=DEV)
+    lse, z = torch.empty_like(top), torch.empty_like(top)
+    for r in range(x.shape[0]):
+        d = x[r].double()
+        top[r] = d.max()
+        z[r] = torch.exp(d - top[r]).sum()
+        lse[r] = top[r] + torch.log(z[r])
+    if kind == "confidence":
+        return {"argmax": None, "max_sumexp": torch.stack([top, z], dim=1), "status": None}
+    token, n = rest
+    out = {"lse": lse, "status": None, "logprob": x.gather(1, token[:, None].long())[:, 0].double() - lse}
+    if n > 0:
+        best = torch.stack([torch.topk(x[r].float(), n).values for r in range(x.shape[0])])
+        out.update(top_id=None, top_logprob=best.double() - lse[:, None])
+    return out
