@@ -25,6 +25,9 @@ __device__ __forceinline__ uint32_t key_of(float v) {
 __device__ __forceinline__ float value_of(uint32_t k) {
   return __uint_as_float((k & 0x80000000u) ? (k ^ 0x80000000u) : ~k);
 }
+// the value from which on a float belongs to keys >= k (a key from a search may lie between the
+// numbers: below that of -inf it stands for -inf, never for a NaN)
+__device__ __forceinline__ float floor_value(uint32_t k) { return k < 0x007FFFFFu ? -INFINITY : value_of(k); }
 // 64-bit composite: larger = better under (value descending, id ascending)
 __device__ __forceinline__ uint64_t comp_of(uint32_t key, int32_t id) {
   return ((uint64_t)key << 32) | (uint32_t)(0xFFFFFFFFu - (uint32_t)id);
@@ -215,6 +218,21 @@ __device__ __forceinline__ uint4 ldg128_stream(const void* p) {
   asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
                : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
                : "l"(p));
+  return r;
+}
+// asks for `bytes` (a multiple of 16, from a 16-byte boundary on) to be brought into the L2 cache
+__device__ __forceinline__ void prefetch_l2(const void* p, int bytes) {
+  asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+}
+// ldg128_stream where `on` holds; elsewhere four words of `fill` (no branch)
+__device__ __forceinline__ uint4 ldg128_stream_if(const void* p, bool on, uint32_t fill) {
+  uint4 r = make_uint4(fill, fill, fill, fill);
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %5, 0;\n\t"
+      "@p ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+      : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w)
+      : "l"(p), "r"((uint32_t)on));
   return r;
 }
 

@@ -1,454 +1,413 @@
 // logprobs_batch: per row the log-softmax of one token and the top_n largest raw logits as log
 // probabilities (tools/server_chat.h:417-441; zero/runz.cpp:478-484 scores perplexity with the
-// same sum). One launch. A CTA streams one segment of one row once through a ring of bulk-copied
-// tiles and keeps
-//  - per thread a running (reference value, sum of exponentials relative to it), the sum in fp64;
-//  - for the whole CTA a candidate buffer with a rising threshold: the top_n best so far.
-// Rows are cut into segments when there are few of them; the CTA that finishes a row last merges
-// the segments' results (left in the workspace) and writes the row's output.
+// same sum). One launch, one pass. The rows, cut into units of columns, are dealt out to the CTAs in
+// equal runs of consecutive units (lp_plan): a CTA takes the end of one row, some whole rows and
+// the beginning of another, so that no wave of CTAs is left half empty and a row is cut only where
+// one CTA's share ends. Every such piece of a row is read once, straight into registers (a tile of
+// four 16-byte chunks a thread, the next tile's loads in flight while one is worked on), and gives
+//  - per thread a sum of exponentials relative to a reference value of the thread's own, in fp64;
+//  - notes of the threads' tiles that may hold one of the top_n largest elements, which are read
+//    again at the piece's end.
+// After a piece's first tile no thread waits for another. The CTA that finishes a row last merges its pieces
+// (left in the workspace) and writes the row's output.
+//
+// What bounds it: memory, then the special-function unit (one ex2 per logit, 16 a clock and SM:
+// 59 us for 1024 x 262144, next to 82 us for its 537 MB); what the kernel takes on top are the pieces'
+// ends and beginnings. 1024 x 262144 bf16: 20 alternatives 226 -> 151 us, none 140 -> 104 us; 512 x 151936
+// fp32, none: 84 -> 57 us (a CTA per row through a shared-memory ring with two barriers a tile, the
+// candidates' buffer kept by the whole CTA, -> this).
+#include <algorithm>
+
 #include "plan.h"
 #include "select.cuh"
 #include "stream.cuh"
 
 namespace arcs {
 
+constexpr int kLpThreads = 128;               // threads of a CTA
 constexpr int kLpCap = 1024;                  // candidate buffer of a CTA
-constexpr int kLpTrig = kLpCap - kThreads;    // prune once it has grown past this
-constexpr int kLpPerSm = 3;                   // CTAs per SM the segments are planned for
+constexpr int kLpTrig = kLpCap - kLpThreads;    // prune once it has grown past this
+// CTAs per SM the work is dealt out to. With alternatives five, which leaves the compiler enough
+// registers (64 alternatives 185 -> 169 us, 256: 433 -> 287 us); without them six (111 -> 105 us).
+__host__ __device__ constexpr int lp_per_sm(bool top) { return top ? 5 : 6; }
+constexpr int kLpChunks = 4;                  // 16-byte chunks a thread holds of one tile
+constexpr int kLpTileBytes = kLpChunks * kLpThreads * 16;
+constexpr int kLpAhead = 3;                   // tiles ahead of the one worked on that are asked into the L2 cache
+constexpr int kLpFew = 64;                    // up to so many alternatives one maximum per thread gives a tight threshold
+// records a CTA keeps of threads and tiles whose maximum reached the threshold of the moment: one a thread of
+// the first tile, then about as many as alternatives wanted (plus a seventh) each time the piece doubles
+template <int TOP> constexpr int kLpRec = TOP == 0 ? 1 : TOP == 1 ? 1024 : 3072;
 
-struct LpPart {      // what a segment leaves for the merge
-  double z;          // sum of exp(l - M) over the segment
-  float M;           // the segment's maximum (-inf: nothing but NaN or -inf)
+struct LpPart {      // what a piece leaves for the merge
+  double z;          // sum of exp(l - M) over the piece
+  float M;           // the largest of its threads' references (-inf: nothing but NaN or -inf)
   int32_t cnt;       // entries in its candidate list
 };
 
 struct LogprobDev {
   const void* logits;
   int64_t row_stride;
-  int32_t B, V, nseg, seg_len;
+  int32_t B, V;
+  int32_t unit, row_units;         // columns per unit, units per row
+  uint32_t run, longer;            // units every CTA takes, CTAs that take one more (the first ones)
+  int32_t max_pieces;              // pieces a row can be cut into
   const int32_t* token;
   int32_t top_n, top_stride;
   double* logprob;
   double* lse;
   int32_t* top_id;
   double* top_logprob;
-  unsigned int* ws_ctr;            // [B] segments of the row that have finished, 0 between launches
-  LpPart* ws_part;                 // [B][nseg]
-  unsigned long long* ws_list;     // [B][nseg][top_n] composites
+  unsigned int* ws_ctr;            // [B] pieces of the row that have finished, 0 between launches
+  LpPart* ws_part;                 // [B][max_pieces]
+  unsigned long long* ws_list;     // [B][max_pieces][n] composites
   int32_t* status;
 };
 
-// exp(v - m) for v <= m as 2^((v - m) * log2 e) by the special-function unit. Measured against
-// fp64 sums the log of a row's sum comes out within 4e-8 whatever is done about the roundings of
-// the difference and of the product (first-order corrections were tried: the unit's own error
-// dominates), so nothing is. NaN and -inf give 0.
-__device__ __forceinline__ float exp_diff(float v, float m) {
-  constexpr float kL2e = 1.44269502162933349609375f;
+constexpr float kL2e = 1.44269502162933349609375f;  // log2 e rounded to fp32
+
+__device__ __forceinline__ float ex2(float x) {
   float e;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(__fmul_rn(__fsub_rn(fmaxf(v, -1e38f), m), kL2e)));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x));
   return e;
 }
-
-// Warp-collective append to the candidate buffer; lanes with p set store (key, id). Returns true
-// for a lane whose entry found no room (the caller offers it again after the next prune); `hot`
-// is set once the buffer has grown past the prune trigger.
-__device__ __forceinline__ bool lp_push(const Sel& s, bool p, uint32_t key, int32_t id, bool& hot) {
-  const unsigned b = __ballot_sync(0xFFFFFFFFu, p);
-  if (b == 0) return false;
-  const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
-  int base = 0;
-  if (lane == leader) base = (int)sm_atomic_add(s.cnt, (uint32_t)__popc(b));
-  base = __shfl_sync(0xFFFFFFFFu, base, leader);
-  if (!p) return false;
-  const int pos = base + __popc(b & ((1u << lane) - 1u));
-  hot = hot || pos + 1 > s.trig;
-  if (pos >= s.cap) return true;
-  s.key[pos] = key;
-  s.id[pos] = id;
-  return false;
+// a float that is neither negative, infinite nor NaN, widened by integer operations (the conversion
+// instruction shares the special-function unit with the exponentials; zero comes out as 2^-127)
+__device__ __forceinline__ double widen_pos(float x) {
+  const uint32_t b = __float_as_uint(x);
+  return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
 }
 
-constexpr size_t kLpSmem = (size_t)kStages * kTileBytes + (size_t)kLpCap * 8 + 512 * 4 + (size_t)kTmpCap * 8;
+// the largest element of several chunks (NaN ignored), a chunk of -inf
+template <typename T> struct LpElem;
+template <> struct LpElem<float> {
+  static constexpr uint32_t kNothing = 0xFF800000u;
+  static __device__ __forceinline__ float tile_max(const uint4 (&q)[kLpChunks]) {
+    float m = Elem<float>::chunk_max(q[0]);
+#pragma unroll
+    for (int j = 1; j < kLpChunks; ++j) m = fmaxf(m, Elem<float>::chunk_max(q[j]));
+    return m;
+  }
+};
+template <> struct LpElem<__nv_bfloat16> {
+  static constexpr uint32_t kNothing = 0xFF80FF80u;
+  static __device__ __forceinline__ float tile_max(const uint4 (&q)[kLpChunks]) {
+    __nv_bfloat162 m[kLpChunks];
+#pragma unroll
+    for (int j = 0; j < kLpChunks; ++j) {
+      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&q[j]);
+      m[j] = __hmax2(__hmax2(p[0], p[1]), __hmax2(p[2], p[3]));  // NaN-ignoring packed max
+    }
+#pragma unroll
+    for (int w = kLpChunks / 2; w > 0; w >>= 1)
+#pragma unroll
+      for (int j = 0; j < w; ++j) m[j] = __hmax2(m[j], m[j + w]);
+    return fmaxf(__low2float(m[0]), __high2float(m[0]));
+  }
+};
 
+// A thread's running sum of exponentials: S * 2^c = sum of 2^(l * kL2e) over what it has seen, c
+// the rounded product ref * kL2e. A term is ex2(fma(l, kL2e, -c)): one rounding, and c's own is
+// made good once, when the sum is taken (scaled()). The terms of a chunk are added in fp32, the
+// chunks in fp64. The reference is at least every element the thread has seen: the terms that make
+// up a peaked sum are exact ones. Against fp64 sums the log of a row's sum has an rms error of
+// 0.9e-8 (fp32 normal logits, 512 rows of 151936; 1.1e-8 when exponents were rounded twice).
+struct LpSum {
+  float ref = -INFINITY, c = -INFINITY;
+  double S = 0.0;
+  __device__ __forceinline__ double off() const { return (double)ref * (double)kL2e - (double)c; }  // exact: what the terms' exponents are short of
+  __device__ __forceinline__ double scaled() const { return S == 0.0 ? 0.0 : S * exp2(-off()); }    // sum of exp(l - ref)
+  // a new, larger reference
+  __device__ __forceinline__ void raise(float m) {
+    const float cm = __fmul_rn(m, kL2e);
+    if (S != 0.0) S *= exp2((double)c - (double)cm);
+    ref = m;
+    c = cm;
+  }
+  // one more value, in the slow way
+  __device__ __forceinline__ void one(float v) {
+    if (v > ref) raise(v);
+    if (ref > -INFINITY && v == v) S += exp((double)v - (double)ref) * exp2(off());
+  }
+};
+// The rare steps of the main loop are calls: what they need in registers is then spilled around
+// them and not in the loop itself.
+__device__ __noinline__ double lp_rescale(double S, float c, float cm) { return S * exp2((double)c - (double)cm); }
+// (the thread's chunks first, first + kLpThreads, ... of a piece with nchunk of them at body, read once more)
 template <typename T>
-__global__ void __launch_bounds__(kThreads) logprob_kernel(const LogprobDev a) {
-  extern __shared__ __align__(128) char smem[];
-  char* stage = smem;
-  uint32_t* bkey = reinterpret_cast<uint32_t*>(smem + (size_t)kStages * kTileBytes);
-  int32_t* bid = reinterpret_cast<int32_t*>(bkey + kLpCap);
-  uint32_t* hist = reinterpret_cast<uint32_t*>(bid + kLpCap);
-  uint32_t* tk = hist + 512;
-  int32_t* ti = reinterpret_cast<int32_t*>(tk + kTmpCap);
-  __shared__ __align__(8) uint64_t bars[kStages];
-  __shared__ unsigned long long s_tau, s_m64;
-  __shared__ int s_cnt, s_misc[8], s_flag;
-  __shared__ uint32_t s_maxkey;
-  __shared__ float red_m[kThreads / 32];
-  __shared__ double red_s[kThreads / 32], s_lse;
-  __shared__ __align__(16) uint32_t s_keys[kThreads];
+__device__ __noinline__ double lp_tile_slow(double S, float ref, float c, const char* body, int first, int nchunk) {
+  LpSum s;
+  s.S = S;
+  s.ref = ref;
+  s.c = c;
+  const int end = min(nchunk, first + kLpChunks * kLpThreads);
+  for (int i = first; i < end; i += kLpThreads) {
+    const uint4 q = ldg128_stream(body + (size_t)i * 16);
+#pragma unroll
+    for (int e = 0; e < Elem<T>::kPerChunk; ++e) s.one(Elem<T>::get(q, e));  // (none exceeds the reference)
+  }
+  return s.S;
+}
+// What the threads have published of their own maxima belongs to disjoint sets of elements, so the
+// n-th largest of it is a lower bound of the n-th largest element: the threshold (a key,
+// inclusive, 16-bit resolution) rises to it. One warp calls.
+template <int PER>
+__device__ __noinline__ void lp_raise_threshold(const uint32_t* keys, int n, uint32_t* tkey) {
+  const uint32_t k = warp_kth16<PER>(keys, n);
+  if ((threadIdx.x & 31) == 0) asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(smem_addr(tkey)), "r"(k) : "memory");
+}
 
+// The n best of a piece read once more, element by element (slow, and rare: the chunks set aside
+// overflowed, with ascending data or masses of equal logits). Called by all threads.
+template <typename T>
+__device__ __noinline__ void lp_reread(const SegPlan& p, const T* row, const Sel& sel, const PruneScratch& ps) {
   constexpr int E = Elem<T>::kPerChunk;
-  constexpr int kChunks = kTileBytes / 16 / kThreads;
-  static_assert(kChunks * E <= 32, "a thread's elements of one tile are tracked in a 32-bit mask");
-  const int tid = threadIdx.x, b = blockIdx.x / a.nseg, seg = blockIdx.x % a.nseg;
-  const T* row = reinterpret_cast<const T*>(a.logits) + (size_t)b * a.row_stride;
-  const int32_t lo = seg * a.seg_len, hi = min(a.V, lo + a.seg_len);
-  const SegPlan p = make_plan(row, lo, hi);
-  const int n = min(a.top_n, a.V);
-
-  Sel sel{bkey, bid, &s_cnt, &s_tau, n, kLpTrig, kLpCap};
-  PruneScratch ps{hist, tk, ti, s_misc, &s_m64};
-
+  const int tid = threadIdx.x, nchunk = p.body_bytes / 16;
+  __syncthreads();
   if (tid == 0) {
-    for (int i = 0; i < kStages; ++i) mbar_init(&bars[i], 1);
-    mbar_init_fence();
-    s_cnt = 0;
-    s_tau = 0ull;
+    *sel.cnt = 0;
+    *sel.tau = 0ull;
   }
   __syncthreads();
-  if (tid == 0)
-    for (int t = 0; t < p.tiles && t < kStages; ++t) issue_tile(p, t, stage, bars);
-
-  float lm = -INFINITY;  // what this thread's exponentials are relative to: at least every value it has seen
-  double ls = 0.0;
-  float own = -INFINITY;  // the largest value this thread itself has seen
-  unsigned long long tau = 0ull;  // exclusive threshold of the candidate buffer (every thread's copy is current)
-
-  // one more value for the sum
-  auto lse_one = [&](float v) {
-    own = fmaxf(own, v);
-    if (v > lm) {
-      ls *= exp((double)lm - (double)v);
-      lm = v;
-    }
-    if (lm > -INFINITY) ls += (double)exp_diff(v, lm);
-  };
-  // All threads call. The threads' own maxima belong to disjoint sets of elements, so the n-th
-  // largest of them is a lower bound of the n-th largest element: the threshold rises to it
-  // without a look at the buffer (16-bit key resolution, one warp). The largest of them becomes
-  // every thread's reference for its exponentials: a thread then meets a larger value, and pays
-  // for the fp64 rescaling of its sum, only where the CTA as a whole does.
-  auto share_maxima = [&](bool reference) {
-    __syncthreads();  // (s_keys may still be read from the last time)
-    s_keys[tid] = own > -INFINITY ? key_of(own) : 0u;
-    __syncthreads();
-    if (tid < 32) {
-      uint32_t mk = 0;
-#pragma unroll
-      for (int i = 0; i < kThreads / 32; ++i) mk = max(mk, s_keys[i * 32 + tid]);
-      mk = __reduce_max_sync(0xFFFFFFFFu, mk);
-      const uint32_t k = n > 0 ? warp_kth16<kThreads / 32>(s_keys, n) : 0u;
-      const unsigned long long cand = k ? ((unsigned long long)k << 32) - 1ull : 0ull;
-      if (tid == 0) {
-        s_maxkey = mk;
-        if (cand > s_tau) s_tau = cand;
-      }
-    }
-    __syncthreads();
-    tau = s_tau;
-    if (reference && s_maxkey != 0u) {
-      const float top = value_of(s_maxkey);
-      if (top > lm) {
-        ls *= exp((double)lm - (double)top);
-        lm = top;
-      }
-    }
-  };
-  // A lane sets the (few) elements it finds above the threshold aside, two at most, and the warp
-  // appends what its lanes hold to the buffer in one go, now and then: an append costs the warp
-  // a round trip to a shared counter.
-  uint32_t sk0 = 0, sk1 = 0;
-  int32_t si0 = 0, si1 = 0;
-  int ns = 0;
-  bool hot = false;
-  auto warp_flush = [&]() {
-    const bool lost1 = lp_push(sel, ns == 2 && comp_of(sk1, si1) > tau, sk1, si1, hot);
-    if (ns == 2 && !lost1) ns = 1;
-    const bool lost0 = lp_push(sel, ns == 1 && comp_of(sk0, si0) > tau, sk0, si0, hot);
-    if (ns == 1 && !lost0) ns = 0;
-  };
-  // Every thread calls with the mask of its own elements that may belong to the n best;
-  // elem(idx, key, id) names element idx. `flush`: what the lanes hold goes to the buffer before
-  // the call returns. When the buffer has grown past the trigger, or had no room for some entry,
-  // the CTA keeps the n best, the threshold rises and what was left out is offered again.
-  auto push_all = [&](uint32_t bits, bool flush, auto elem) {
-    uint32_t again = 0;
-    for (;;) {
-      while (__any_sync(0xFFFFFFFFu, bits != 0u)) {
-        if (__any_sync(0xFFFFFFFFu, bits != 0u && ns == 2)) warp_flush();
-        if (bits != 0u) {
-          const int idx = __ffs(bits) - 1;
-          bits &= bits - 1u;
-          if (ns < 2) {
-            uint32_t ky = 0;
-            int32_t id = 0;
-            elem(idx, ky, id);
-            if (ky != 0u && comp_of(ky, id) > tau) {
-              if (ns == 0) {
-                sk0 = ky;
-                si0 = id;
-              } else {
-                sk1 = ky;
-                si1 = id;
-              }
-              ++ns;
-            }
-          } else {
-            again |= 1u << idx;  // (the buffer is full: after the prune)
-          }
-        }
-      }
-      if (flush) warp_flush();
-      if (!__syncthreads_or(hot || again != 0u || (flush && ns > 0))) break;
-      const unsigned long long before = tau;
-      sel_prune<1, kThreads>(sel, n, ps, tid);
-      if (s_tau < before) {  // (entries still held by lanes were not in the buffer: its n-th best may lie below the threshold)
-        __syncthreads();
-        if (tid == 0) s_tau = before;
-        __syncthreads();
-      }
-      tau = s_tau;
-      hot = false;
-      bits = again;
-      again = 0;
-    }
-  };
-
-  bool failed = false;
-  for (int t = 0; t < p.tiles; ++t) {
-    const int slot = t % kStages;
-    if (!mbar_wait(&bars[slot], (uint32_t)((t / kStages) & 1))) failed = true;
-    const uint32_t nbytes = tile_bytes(p, t);
-    uint4 q[kChunks];
-#pragma unroll
-    for (int j = 0; j < kChunks; ++j) {
-      const uint32_t off = (uint32_t)(j * kThreads + tid) * 16u;
-      q[j] = off < nbytes && !failed ? lds128(stage + (size_t)slot * kTileBytes + off) : make_uint4(0, 0, 0, 0);
-    }
-    // every thread has taken its chunks: the slot can be refilled
-    if (__syncthreads_or(failed)) {
-      if (tid == 0) {
-        raise_status(a.status, ARCS_ERR_TIMEOUT);
-        drain_tiles(p, t, bars);
-      }
-      __syncthreads();
-      return;
-    }
-    if (tid == 0 && t + kStages < p.tiles) issue_tile(p, t + kStages, stage, bars);
-
-    // ---- the sum of exponentials
-    float cmax[kChunks];
-#pragma unroll
-    for (int j = 0; j < kChunks; ++j) {
-      const uint32_t off = (uint32_t)(j * kThreads + tid) * 16u;
-      cmax[j] = NAN;  // (a chunk past the end of the tile reaches no threshold, not even -inf)
-      if (off >= nbytes) continue;
-      const float cm = Elem<T>::chunk_max(q[j]);
-      cmax[j] = cm;
-      own = fmaxf(own, cm);
-      if (cm > lm) {
-        ls *= exp((double)lm - (double)cm);
-        lm = cm;
-      }
-      if (lm > -INFINITY) {
-        float ev[E];
-#pragma unroll
-        for (int e = 0; e < E; ++e) ev[e] = exp_diff(Elem<T>::get(q[j], e), lm);
-#pragma unroll
-        for (int w = E / 2; w > 0; w >>= 1)
-#pragma unroll
-          for (int e = 0; e < w; ++e) ev[e] += ev[e + w];
-        ls += (double)ev[0];
-      }
-    }
-    if (t == 0 || t == 3 || t == 15 || t == 63) share_maxima(true);
-    if (n <= 0) continue;
-
-    // ---- the candidates
-    const int32_t tile_first = p.body_first + (int32_t)((uint32_t)t * kTileBytes / sizeof(T));
-    const uint32_t tkey = (uint32_t)(tau >> 32);
-    const float tf = value_of(tkey < 0x007FFFFFu ? 0x007FFFFFu : tkey);  // inclusive value threshold
-    // the chunks whose maximum reaches the threshold are few: only they are looked into, in a
-    // loop the warp leaves as soon as no lane has one; what passes is set aside by the lane
-    uint32_t hotc = 0;
-#pragma unroll
-    for (int j = 0; j < kChunks; ++j) hotc |= (cmax[j] >= tf ? 1u : 0u) << j;
+  for (int c0 = 0; c0 < nchunk; c0 += kLpChunks * kLpThreads) {
+    uint4 q[kLpChunks];
     uint32_t bits = 0;
-    while (__any_sync(0xFFFFFFFFu, hotc != 0u)) {
-      if (hotc != 0u) {
-        const int j = __ffs(hotc) - 1;
-        hotc &= hotc - 1u;
-        uint4 c = q[0];
+    const uint32_t tkey = (uint32_t)(*sel.tau >> 32);
 #pragma unroll
-        for (int x = 1; x < kChunks; ++x)
-          if (j == x) c = q[x];
-        const int32_t id0 = tile_first + (int32_t)((uint32_t)(j * kThreads + tid) * 16u / sizeof(T));
+    for (int j = 0; j < kLpChunks; ++j) {
+      const int ci = c0 + j * kLpThreads + tid;
+      q[j] = ci < nchunk ? ldg128_stream(p.body + (size_t)ci * 16) : make_uint4(0, 0, 0, 0);
 #pragma unroll
-        for (int e = 0; e < E; ++e) {
-          const float v = Elem<T>::get(c, e);
-          if (v >= tf) {
-            const uint32_t ky = key_of(v);
-            if (ky != 0u && comp_of(ky, id0 + e) > tau) {
-              if (ns == 0) {
-                sk0 = ky;
-                si0 = id0 + e;
-                ns = 1;
-              } else if (ns == 1) {
-                sk1 = ky;
-                si1 = id0 + e;
-                ns = 2;
-              } else {
-                bits |= 1u << (j * E + e);  // (no room in the lane: the general path below)
-              }
-            }
-          }
-        }
-      }
+      for (int e = 0; e < E; ++e) bits |= (ci < nchunk && key_of(Elem<T>::get(q[j], e)) >= tkey ? 1u : 0u) << (j * E + e);
     }
-    push_all(bits, (t & 7) == 7 || t + 1 == p.tiles, [&](int idx, uint32_t& ky, int32_t& id) {
+    push_all<kLpThreads>(sel, ps, bits, [&](int idx, uint32_t& ky, int32_t& id) {
       const int j = idx / E;
       uint4 c = q[0];
 #pragma unroll
-      for (int x = 1; x < kChunks; ++x)
+      for (int x = 1; x < kLpChunks; ++x)
         if (j == x) c = q[x];
-      id = tile_first + (int32_t)((uint32_t)(j * kThreads + tid) * 16u / sizeof(T)) + idx % E;
+      id = p.body_first + (c0 + j * kLpThreads + tid) * E + idx % E;
       ky = key_of(Elem<T>::get(c, idx % E));
     });
   }
+  const bool hv = tid < p.head_n, tv = tid < p.tail_n;
+  push_all<kLpThreads>(sel, ps, (hv ? 1u : 0u) | (tv ? 2u : 0u), [&](int idx, uint32_t& ky, int32_t& id) {
+    id = idx == 0 ? p.lo + tid : p.tail_first + tid;
+    ky = key_of(Elem<T>::load(row + id));
+  });
+}
 
-  // ---- the few elements outside the 16-byte aligned body
-  {
-    const bool hv = tid < p.head_n, tv = tid < p.tail_n;
-    const float vh = hv ? Elem<T>::load(row + lo + tid) : 0.0f;
-    const float vt = tv ? Elem<T>::load(row + p.tail_first + tid) : 0.0f;
-    if (hv) lse_one(vh);
-    if (tv) lse_one(vt);
-    if (n > 0)
-      push_all((hv ? 1u : 0u) | (tv ? 2u : 0u), true, [&](int idx, uint32_t& ky, int32_t& id) {
-        ky = key_of(idx == 0 ? vh : vt);
-        id = idx == 0 ? lo + tid : p.tail_first + tid;
-      });
-  }
+// the first unit of a CTA's run, and the CTA whose run holds a unit
+__host__ __device__ inline uint32_t lp_first_unit(uint32_t cta, uint32_t run, uint32_t longer) { return cta * run + (cta < longer ? cta : longer); }
+__host__ __device__ inline uint32_t lp_cta_of(uint32_t u, uint32_t run, uint32_t longer) {
+  const uint32_t split = longer * (run + 1);
+  return u < split ? u / (run + 1) : longer + (u - split) / run;
+}
 
-  // the CTA's (maximum, sum of exponentials relative to it) from the threads' pairs; the sum is
-  // returned to thread 0
-  auto cta_lse = [&](float m_t, double s_t, float& M) -> double {
-    M = m_t;
+// what the threads of a CTA share
+template <int TOP>
+struct LpShared {
+  static constexpr int OWN = TOP == 2 ? kLpChunks : 1;  // maxima a thread keeps
+  unsigned long long tau, m64;
+  double red_s[kLpThreads / 32], lse;
+  alignas(16) uint32_t keys[TOP ? OWN * kLpThreads : 4];  // what the threads publish of their maxima (read four at a time)
+  float rec_max[kLpRec<TOP>];                           // threads' maxima of tiles that reached the threshold
+  uint32_t rec_at[kLpRec<TOP>];                         // ... tile << 8 | thread
+  uint32_t bkey[TOP ? kLpCap : 1];                      // the piece's candidates
+  int32_t bid[TOP ? kLpCap : 1];
+  uint32_t hist[TOP ? 512 : 1];
+  uint32_t tk[TOP ? kTmpCap : 1];
+  int32_t ti[TOP ? kTmpCap : 1];
+  float red_m[kLpThreads / 32];
+  uint32_t wkey[kLpThreads / 32];
+  uint32_t tkey;                                        // the threshold (a key, inclusive)
+  int rec, cnt, misc[8], flag, cnts[kMaxSeg];
+};
+
+// The end of a piece (columns of units s0 .. s1 of row b): its sum and candidates, the merge of the
+// row's pieces, the row's output. ref, z: the thread's sum. Called by all threads; a function of its
+// own, so that the main loop's registers are not spilled for it.
+template <typename T, int TOP>
+__device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, int b, int s0, int s1, int tiles, float M, double z) {
+  constexpr int E = Elem<T>::kPerChunk;
+  constexpr int OWN = LpShared<TOP>::OWN;
+  const int tid = threadIdx.x;
+  const int n = TOP ? min(a.top_n, a.V) : 0;
+  const Sel sel{sh.bkey, sh.bid, &sh.cnt, &sh.tau, n, kLpTrig, kLpCap};
+  const PruneScratch ps{sh.hist, sh.tk, sh.ti, sh.misc, &sh.m64};
+  const T* row = reinterpret_cast<const T*>(a.logits) + (size_t)b * a.row_stride;
+  const SegPlan p = make_plan(row, s0 * a.unit, min(a.V, s1 * a.unit));
+  const int nchunk = p.body_bytes / 16;
+  const bool hv = tid < p.head_n, tv = tid < p.tail_n;
+  const float vh = TOP && hv ? Elem<T>::load(row + p.lo + tid) : -INFINITY;
+  const float vt = TOP && tv ? Elem<T>::load(row + p.tail_first + tid) : -INFINITY;
+  // a warp's (reference, sum of exponentials relative to it) from its lanes' pairs, and the CTA's from
+  // its warps' (left in sh.red_m / sh.red_s; called by warp 0)
+  auto warp_lse = [&](float& m, double& z) {
+    float M = m;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) M = fmaxf(M, __shfl_xor_sync(0xFFFFFFFFu, M, o));
-    __syncthreads();  // (red_m / red_s may still be read from an earlier call)
-    if ((tid & 31) == 0) red_m[tid >> 5] = M;
-    __syncthreads();
-    M = red_m[0];
+    z = m > -INFINITY ? z * exp((double)m - (double)M) : 0.0;
 #pragma unroll
-    for (int w = 1; w < kThreads / 32; ++w) M = fmaxf(M, red_m[w]);
-    double part = m_t > -INFINITY ? s_t * exp((double)m_t - (double)M) : 0.0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) part += __shfl_xor_sync(0xFFFFFFFFu, part, o);
-    if ((tid & 31) == 0) red_s[tid >> 5] = part;
-    __syncthreads();
-    double z = 0.0;
-    if (tid == 0)
-      for (int w = 0; w < kThreads / 32; ++w) z += red_s[w];
-    return z;
+    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xFFFFFFFFu, z, o);
+    m = M;
   };
-  float M;
-  double z = cta_lse(lm, ls, M);
-  // What is left of the buffer once a last threshold (from the threads' own maxima, where the
-  // buffer holds this CTA's own elements) has been applied: a little more than n entries as a
-  // rule. Where the n best are needed, an entry's place is the number of entries above it
-  // (composites are unique).
-  auto settle = [&](bool own_elements) -> int {
-    if (own_elements) share_maxima(false);
-    else __syncthreads();
-    const int c0 = min(s_cnt, kLpCap);
-    unsigned long long mine[kLpCap / kThreads];
-#pragma unroll
-    for (int x = 0; x < kLpCap / kThreads; ++x) {
-      const int i = tid + x * kThreads;
-      mine[x] = i < c0 ? comp_of(bkey[i], bid[i]) : 0ull;
-    }
-    __syncthreads();
-    if (tid == 0) s_cnt = 0;
-    __syncthreads();
-    bool hot = false;
-#pragma unroll
-    for (int x = 0; x < kLpCap / kThreads; ++x) lp_push(sel, mine[x] > tau, comp_key(mine[x]), comp_id(mine[x]), hot);
-    __syncthreads();
-    if (s_cnt > 512) {
-      sel_prune<1, kThreads>(sel, n, ps, tid);
-      __syncthreads();
-    }
-    return min(s_cnt, kLpCap);
+  auto cta_lse = [&](float& m, double& z) {
+    const int w = tid & 31;
+    m = w < kLpThreads / 32 ? sh.red_m[w] : -INFINITY;
+    z = w < kLpThreads / 32 ? sh.red_s[w] : 0.0;
+    warp_lse(m, z);
   };
-  auto rank_of = [&](int i, int c) -> int {
-    const uint64_t ci = comp_of(bkey[i], bid[i]);
+  auto rank_of = [&](int i, int c) -> int {  // composites are unique: an entry's place is the number of entries above it
+    const uint64_t ci = comp_of(sh.bkey[i], sh.bid[i]);
     int rank = 0;
-    for (int j = 0; j < c; ++j) rank += comp_of(bkey[j], bid[j]) > ci;
+    for (int j = 0; j < c; ++j) rank += comp_of(sh.bkey[j], sh.bid[j]) > ci;
     return rank;
   };
 
-  if (a.nseg > 1) {
-    // ---- leave the segment's results; the CTA that finishes the row last merges them
-    const size_t slot = (size_t)b * a.nseg + seg;
-    const int c = n > 0 ? settle(true) : 0, m = min(c, n);
-    for (int i = tid; i < c; i += kThreads) {
+  // ---- the piece's sum, and its candidates: a last threshold, and the elements of the tiles noted
+  // that reach it to the buffer (a little more than n as a rule); afterwards sh.bkey / sh.bid hold c
+  // entries, the n best among them
+  warp_lse(M, z);
+  if ((tid & 31) == 0) {
+    sh.red_m[tid >> 5] = M;
+    sh.red_s[tid >> 5] = z;
+  }
+  if (TOP) {
+  }
+  if (tid == 0) sh.cnt = sh.misc[0] = 0;
+  __syncthreads();
+  if (TOP && tid < 32) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
+  if (TOP) __syncthreads();
+  if (tid < 32) cta_lse(M, z);
+  int c = 0;
+  if (TOP) {
+    const uint32_t tkey = sh.tkey;
+    const float tf = floor_value(tkey);
+    const int have = tiles > 0 ? sh.rec : 0;
+    if (have <= kLpRec<TOP>) {
+      // the records that reach it, closed up (in place: a round's are all read before any is
+      // written, at or before the round's first place)
+      for (int i0 = 0; i0 < have; i0 += kLpThreads) {
+        const int i = i0 + tid;
+        const bool in = i < have && sh.rec_max[i] >= tf;
+        const uint32_t at = i < have ? sh.rec_at[i] : 0u;
+        __syncthreads();
+        if (in) sh.rec_at[sm_atomic_add(&sh.misc[0], 1u)] = at;
+      }
+      __syncthreads();
+      auto keep = [&](float v, int32_t id) {
+        const uint32_t ky = key_of(v);
+        if (!(v >= tf) || ky == 0u) return;
+        const uint32_t at = sm_atomic_add(&sh.cnt, 1u);
+        if (at < (uint32_t)kLpCap) {
+          sh.bkey[at] = ky;
+          sh.bid[at] = id;
+        }
+      };
+      for (int i = tid; i < sh.misc[0] * kLpChunks; i += kLpThreads) {  // (a chunk to a thread, from the L2 cache as a rule)
+        const uint32_t r = sh.rec_at[i / kLpChunks];
+        const int ci = ((int)(r >> 8) * kLpChunks + i % kLpChunks) * kLpThreads + (int)(r & 255u);
+        if (ci >= nchunk) continue;
+        const uint4 ch = ldg128_stream(p.body + (size_t)(uint32_t)ci * 16);
+        if (!(Elem<T>::chunk_max(ch) >= tf)) continue;
+#pragma unroll
+        for (int e = 0; e < E; ++e) keep(Elem<T>::get(ch, e), p.body_first + ci * E + e);
+      }
+      if (hv) keep(vh, p.lo + tid);
+      if (tv) keep(vt, p.tail_first + tid);
+    }
+    __syncthreads();
+    if (have > kLpRec<TOP> || sh.cnt > kLpCap) lp_reread<T>(p, row, sel, ps);
+    if (sh.cnt > 512) {
+      __syncthreads();
+      sel_prune<1, kLpThreads>(sel, n, ps, tid);
+      __syncthreads();
+    }
+    c = min(sh.cnt, kLpCap);
+  }
+
+  const uint32_t row_u = (uint32_t)b * (uint32_t)a.row_units;
+  const int cta0 = (int)lp_cta_of(row_u, a.run, a.longer);
+  const int pieces = (int)lp_cta_of(row_u + (uint32_t)a.row_units - 1u, a.run, a.longer) - cta0 + 1;
+  const int piece = (int)blockIdx.x - cta0;
+  if (pieces > 1) {
+    // ---- leave the piece's results; the CTA that finishes the row last merges them
+    const size_t slot = (size_t)b * a.max_pieces + piece;
+    for (int i = tid; i < c; i += kLpThreads) {
       const int rank = rank_of(i, c);
-      if (rank < n) a.ws_list[slot * n + rank] = comp_of(bkey[i], bid[i]);
+      if (rank < n) a.ws_list[slot * n + rank] = comp_of(sh.bkey[i], sh.bid[i]);
     }
     if (tid == 0) {
       LpPart pt;
       pt.z = z;
       pt.M = M;
-      pt.cnt = m;
+      pt.cnt = min(c, n);
       a.ws_part[slot] = pt;
     }
     __threadfence();
     __syncthreads();
     if (tid == 0) {
-      s_flag = atomicAdd(&a.ws_ctr[b], 1u) == (unsigned)a.nseg - 1u;
-      if (s_flag) a.ws_ctr[b] = 0u;  // left at zero for the next launch
+      sh.flag = atomicAdd(&a.ws_ctr[b], 1u) == (unsigned)pieces - 1u;
+      if (sh.flag) a.ws_ctr[b] = 0u;  // left at zero for the next launch
     }
     __syncthreads();
-    if (!s_flag) return;
+    if (!sh.flag) return;  // (every warp is past its reads of the shared arrays, but for sh.flag: written again behind two barriers)
     __threadfence();
     float pm = -INFINITY;
     double pz = 0.0;
     int pc = 0;
-    if (tid < a.nseg) {
-      const LpPart* src = &a.ws_part[(size_t)b * a.nseg + tid];
+    if (tid < pieces) {
+      const LpPart* src = &a.ws_part[(size_t)b * a.max_pieces + tid];
       pz = __ldcg(&src->z);
       pm = __ldcg(&src->M);
       pc = __ldcg(&src->cnt);
     }
-    z = cta_lse(pm, pz, M);
-    if (n > 0) {
+    if (TOP) {
+      // A piece that sent n entries has n at or above its last: nothing below the largest such
+      // entry is among the n best of the row.
+      
       if (tid == 0) {
-        s_cnt = 0;
-        s_tau = 0ull;
+        sh.cnt = 0;
+        sh.tau = 0ull;
       }
+      if (tid < pieces) sh.cnts[tid] = pc;
       __syncthreads();
-      tau = 0ull;
-      // the segments' lists go through the buffer, kThreads entries at a time
-      __shared__ int s_cnts[kMaxSeg];
-      if (tid < a.nseg) s_cnts[tid] = pc;
+      if (tid < pieces && pc == n)
+        sm_red_max_u64(&sh.tau, __ldcg(&a.ws_list[((size_t)b * a.max_pieces + tid) * n + n - 1]) - 1ull);
       __syncthreads();
-      for (int e0 = 0; e0 < a.nseg * n; e0 += kThreads) {
-        const int e = e0 + tid, g = e / n, i = e % n;
-        const bool have = e < a.nseg * n && i < s_cnts[g];
-        const unsigned long long c = have ? __ldcg(&a.ws_list[((size_t)b * a.nseg + g) * n + i]) : 0ull;
-        push_all(have ? 1u : 0u, true, [&](int, uint32_t& ky, int32_t& id) {
-          ky = comp_key(c);
-          id = comp_id(c);
+      // the pieces' lists go through the buffer, kLpThreads entries at a time
+      for (int e0 = 0; e0 < pieces * n; e0 += kLpThreads) {
+        const int e = e0 + tid, g = e / max(n, 1), i = e - g * n;
+        const bool have = e < pieces * n && i < sh.cnts[g];
+        const unsigned long long cm = have ? __ldcg(&a.ws_list[((size_t)b * a.max_pieces + g) * n + i]) : 0ull;
+        push_all<kLpThreads>(sel, ps, have ? 1u : 0u, [&](int, uint32_t& ky, int32_t& id) {
+          ky = comp_key(cm);
+          id = comp_id(cm);
         });
       }
+      __syncthreads();
+      if (sh.cnt > 512) sel_prune<1, kLpThreads>(sel, n, ps, tid);
+      __syncthreads();
+      c = min(sh.cnt, kLpCap);
     }
+    static_assert(kMaxSeg <= 64, "the pieces' sums lie with two warps");
+    if (tid < 64) {
+      warp_lse(pm, pz);
+      if ((tid & 31) == 0) {
+        sh.red_m[tid >> 5] = pm;
+        sh.red_s[tid >> 5] = pz;
+      }
+    } else if (tid < 64 + kLpThreads / 32 - 2) {
+      sh.red_m[tid - 62] = -INFINITY;
+    }
+    __syncthreads();
+    if (tid < 32) cta_lse(M, z);
   }
 
   // ---- the row's output
   if (tid == 0) {
     const double lse = (double)M + log(z);  // tools/server_chat.h:422
-    s_lse = lse;
+    sh.lse = lse;
     if (a.lse) a.lse[b] = lse;
     if (a.logprob) {
       const int32_t tok = a.token ? a.token[b] : -1;
@@ -456,15 +415,169 @@ __global__ void __launch_bounds__(kThreads) logprob_kernel(const LogprobDev a) {
       a.logprob[b] = (tok >= 0 && tok < a.V) ? (double)Elem<T>::load(row + tok) - lse : (double)NAN;  // :427
     }
   }
-  if (n <= 0) return;
-  const int c = settle(a.nseg == 1);  // (its barriers also publish s_lse)
-  const double lse = s_lse;
-  for (int i = tid; i < c; i += kThreads) {
-    const int rank = rank_of(i, c);
-    if (rank < n) {
-      a.top_id[(size_t)b * a.top_stride + rank] = bid[i];
-      a.top_logprob[(size_t)b * a.top_stride + rank] = (double)value_of(bkey[i]) - lse;
+  if (TOP) {
+    __syncthreads();
+    const double lse = sh.lse;
+    for (int i = tid; i < c; i += kLpThreads) {
+      const int rank = rank_of(i, c);
+      if (rank < n) {
+        a.top_id[(size_t)b * a.top_stride + rank] = sh.bid[i];
+        a.top_logprob[(size_t)b * a.top_stride + rank] = (double)value_of(sh.bkey[i]) - lse;
+      }
     }
+  }
+}
+
+// TOP: 0 no alternatives, 1 up to kLpFew (a threshold from one maximum a thread), 2 any number (four
+// maxima a thread)
+template <typename T, int TOP>
+__global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kernel(const __grid_constant__ LogprobDev a) {
+  constexpr int E = Elem<T>::kPerChunk;
+  constexpr int OWN = LpShared<TOP>::OWN;
+  static_assert(OWN * kLpThreads < 1024, "the search counts to 1023");
+  static_assert(kLpChunks * E <= 32, "a thread's elements of one tile are tracked in a 32-bit mask");
+  __shared__ __align__(16) LpShared<TOP> sh;
+
+  const int tid = threadIdx.x;
+  const int n = TOP ? min(a.top_n, a.V) : 0;
+  uint32_t u = lp_first_unit(blockIdx.x, a.run, a.longer);
+  const uint32_t u_end = lp_first_unit(blockIdx.x + 1, a.run, a.longer);
+
+  while (u < u_end) {
+    // ---- the next piece
+    const int b = (int)(u / (uint32_t)a.row_units), s0 = (int)(u - (uint32_t)b * (uint32_t)a.row_units);
+    const int s1 = (int)min((uint32_t)a.row_units, (uint32_t)s0 + (u_end - u));
+    u += (uint32_t)(s1 - s0);
+    const T* row = reinterpret_cast<const T*>(a.logits) + (size_t)b * a.row_stride;
+    const SegPlan p = make_plan(row, s0 * a.unit, min(a.V, s1 * a.unit));
+    const int nchunk = p.body_bytes / 16;
+    const char* mine = p.body + (size_t)tid * 16;
+    auto fetch = [&](uint4 (&q)[kLpChunks], int t) {
+      const char* from = mine + (size_t)t * kLpTileBytes;
+      if ((t + 1) * (kLpChunks * kLpThreads) <= nchunk) {
+#pragma unroll
+        for (int j = 0; j < kLpChunks; ++j) q[j] = ldg128_stream(from + j * kLpThreads * 16);
+      } else {
+        const int c0 = t * kLpChunks * kLpThreads + tid;
+#pragma unroll
+        for (int j = 0; j < kLpChunks; ++j) q[j] = ldg128_stream_if(from + j * kLpThreads * 16, c0 + j * kLpThreads < nchunk, LpElem<T>::kNothing);
+      }
+    };
+    if (tid == 0 && p.body_bytes > 0) prefetch_l2(p.body, min(kLpAhead * kLpTileBytes, p.body_bytes));
+    uint4 qa[kLpChunks], qb[kLpChunks];  // the tile being worked on and the next, in turn
+    fetch(qa, 0);
+    const bool hv = tid < p.head_n, tv = tid < p.tail_n;  // the few elements outside the 16-byte aligned body
+    const float vh = hv ? Elem<T>::load(row + p.lo + tid) : -INFINITY;
+    const float vt = tv ? Elem<T>::load(row + p.tail_first + tid) : -INFINITY;
+
+    LpSum sum;
+    float own[OWN];  // the largest values this thread itself has seen
+#pragma unroll
+    for (int i = 0; i < OWN; ++i) own[i] = -INFINITY;
+    auto publish = [&]() {
+#pragma unroll
+      for (int i = 0; i < OWN; ++i) sh.keys[i * kLpThreads + tid] = own[i] > -INFINITY ? key_of(own[i]) : 0u;
+    };
+    if (tid == 0) {
+      sh.rec = kLpThreads;  // (the first tile's records have places of their own)
+      sh.tkey = 0u;
+    }
+
+    const int tiles = (nchunk + kLpChunks * kLpThreads - 1) / (kLpChunks * kLpThreads);
+    int point = 1;  // the next tile after which the threads publish their maxima: 1, 3, 7, 15, ...
+    auto tile = [&](int t, const uint4 (&q)[kLpChunks], uint4 (&nq)[kLpChunks]) {
+      if (t + 1 < tiles) fetch(nq, t + 1);
+      if (tid == 0 && t + kLpAhead < tiles) prefetch_l2(p.body + (size_t)(t + kLpAhead) * kLpTileBytes, min(kLpTileBytes, p.body_bytes - (t + kLpAhead) * kLpTileBytes));
+      const float tm = LpElem<T>::tile_max(q);
+      if (TOP == 2) {
+#pragma unroll
+        for (int j = 0; j < OWN; ++j) own[j] = fmaxf(own[j], Elem<T>::chunk_max(q[j]));
+      } else if (TOP == 1) {
+        own[0] = fmaxf(own[0], tm);
+      }
+      if (t == 0) {
+        // The CTA's largest element so far is every thread's first reference: a thread then meets a
+        // larger one, and pays for the rescaling of its sum, some 32 times a row and not at every
+        // maximum of its own.
+        const uint32_t wk = __reduce_max_sync(0xFFFFFFFFu, tm > -INFINITY ? key_of(tm) : 0u);
+        if ((tid & 31) == 0) sh.wkey[tid >> 5] = wk;
+        if (TOP) {
+          publish();
+          sh.rec_max[tid] = tm;
+          sh.rec_at[tid] = tid;
+        }
+        __syncthreads();
+        uint32_t mk = sh.wkey[0];
+#pragma unroll
+        for (int w = 1; w < kLpThreads / 32; ++w) mk = max(mk, sh.wkey[w]);
+        if (mk != 0u) {
+          sum.ref = value_of(mk);
+          sum.c = __fmul_rn(sum.ref, kL2e);
+        }
+        if (TOP && tid < 32) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
+      } else if (tm > sum.ref) {
+        const float cm = __fmul_rn(tm, kL2e);
+        if (sum.S != 0.0) sum.S = lp_rescale(sum.S, sum.c, cm);
+        sum.ref = tm;
+        sum.c = cm;
+      }
+      // ---- the sum of exponentials
+      {
+        float z[kLpChunks];
+#pragma unroll
+        for (int j = 0; j < kLpChunks; ++j) {
+          float e[E];
+#pragma unroll
+          for (int i = 0; i < E; ++i) e[i] = ex2(fmaf(Elem<T>::get(q[j], i), kL2e, -sum.c));
+#pragma unroll
+          for (int w = E / 2; w > 0; w >>= 1)
+#pragma unroll
+            for (int i = 0; i < w; ++i) e[i] += e[i + w];
+          z[j] = e[0];
+        }
+        if ((z[0] + z[1]) + (z[2] + z[3]) < 1e30f) {
+          sum.S += (widen_pos(z[0]) + widen_pos(z[1])) + (widen_pos(z[2]) + widen_pos(z[3]));
+        } else {
+          sum.S = lp_tile_slow<T>(sum.S, sum.ref, sum.c, p.body, t * kLpChunks * kLpThreads + tid, nchunk);  // (a NaN, an infinity, or nothing but -inf so far)
+        }
+      }
+      // ---- a tile that may hold one of the n best is noted, to be looked into at the piece's end
+      if (TOP && t > 0) {
+        const uint32_t tk0 = sm_ld_volatile(&sh.tkey);
+        if (tm >= floor_value(tk0)) {
+          const uint32_t at = sm_atomic_add(&sh.rec, 1u);
+          if (at < (uint32_t)kLpRec<TOP>) {
+            sh.rec_max[at] = tm;
+            sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
+          }
+        }
+        if (t == point) {
+          // (no barrier: what another warp has not published yet only leaves the threshold lower.
+          //  The warps take turns at raising it.)
+          publish();
+          __syncwarp();
+          if ((tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
+          point = 2 * point + 1;
+        }
+      }
+    };
+    if (u < u_end && tid == 0) {  // (the next row's first tile is asked for in time)
+      const uintptr_t next = (reinterpret_cast<uintptr_t>(row + a.row_stride) + 15) & ~(uintptr_t)15;
+      const int bytes = (int)min((int64_t)kLpTileBytes, (int64_t)a.V * (int)sizeof(T) - 16) & ~15;
+      if (bytes > 0) prefetch_l2(reinterpret_cast<const void*>(next), bytes);
+    }
+    for (int t = 0; t < tiles; t += 2) {
+      tile(t, qa, qb);
+      if (t + 1 < tiles) tile(t + 1, qb, qa);
+    }
+    if (hv) sum.one(vh);
+    if (tv) sum.one(vt);
+    if (TOP) {
+      own[0] = fmaxf(own[0], fmaxf(vh, vt));
+      publish();
+    }
+    lp_close<T, TOP>(a, sh, b, s0, s1, tiles, sum.ref, sum.scaled());
+    __syncthreads();  // (the next piece takes the shared arrays over)
   }
 }
 
@@ -472,14 +585,32 @@ __global__ void __launch_bounds__(kThreads) logprob_kernel(const LogprobDev a) {
 
 using namespace arcs;
 
-static void lp_plan(int32_t B, int32_t V, int* nseg, int* seg_len) { plan_segments(B, V, nseg, seg_len, kLpPerSm); }
+// How B rows of V columns are dealt out: units of `unit` columns (a multiple of 2048, at most
+// kMaxSeg to a row), in equal runs to the CTAs, which all fit the GPU at once. 1024 rows as one CTA
+// each are 1.4 waves of 740; dealt out evenly they are one. A row's units lie with at most
+// max_pieces CTAs.
+struct LpPlan {
+  int32_t unit, row_units, max_pieces;
+  uint32_t run, longer;
+  unsigned grid;
+};
+static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n, bool whole) {
+  LpPlan p;
+  p.unit = std::max(2048, ((V - 1) / kMaxSeg + 2048) / 2048 * 2048);
+  if (whole || (int64_t)B * kMaxSeg > INT32_MAX) p.unit = V;
+  p.row_units = (V + p.unit - 1) / p.unit;
+  const uint32_t total = (uint32_t)B * (uint32_t)p.row_units;
+  p.grid = std::min<uint32_t>(total, kSmCount * lp_per_sm(top_n > 0));
+  p.run = total / p.grid;
+  p.longer = total % p.grid;
+  p.max_pieces = (int32_t)std::min<uint32_t>(p.row_units, ((uint32_t)p.row_units - 1 + p.run - 1) / p.run + 1);
+  return p;
+}
 
 extern "C" size_t arcs_logprobs_workspace_bytes(int32_t B, int32_t V, int32_t top_n) {
   if (B <= 0 || V <= 0 || top_n < 0) return 0;
-  int nseg, seg_len;
-  lp_plan(B, V, &nseg, &seg_len);
-  if (nseg == 1) return 16;  // whole rows: nothing is handed over
-  return 256 + (((size_t)B * 4 + 255) & ~(size_t)255) + (size_t)B * nseg * sizeof(LpPart) + (size_t)B * nseg * (size_t)top_n * 8;
+  const LpPlan p = lp_plan(B, V, top_n, false);
+  return 256 + (((size_t)B * 4 + 255) & ~(size_t)255) + (size_t)B * p.max_pieces * (sizeof(LpPart) + (size_t)top_n * 8);
 }
 
 extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
@@ -495,7 +626,16 @@ extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
   a.row_stride = g->row_stride;
   a.B = g->B;
   a.V = g->V;
-  lp_plan(g->B, g->V, &a.nseg, &a.seg_len);
+  // (444 rows or more, or short rows: served without a workspace too, a row to a unit)
+  int nseg, seg_len;
+  plan_segments(g->B, g->V, &nseg, &seg_len, 3);
+  const bool no_ws = nseg == 1 && (!g->workspace || g->workspace_bytes < arcs_logprobs_workspace_bytes(g->B, g->V, g->top_n));
+  const LpPlan plan = lp_plan(g->B, g->V, g->top_n, no_ws);
+  a.unit = plan.unit;
+  a.row_units = plan.row_units;
+  a.run = plan.run;
+  a.longer = plan.longer;
+  a.max_pieces = plan.max_pieces;
   a.token = g->token;
   a.top_n = g->top_n;
   a.top_stride = g->top_stride;
@@ -507,7 +647,7 @@ extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
   a.ws_ctr = nullptr;
   a.ws_part = nullptr;
   a.ws_list = nullptr;
-  if (a.nseg > 1) {
+  if (!no_ws) {
     if (!g->workspace || g->workspace_bytes < arcs_logprobs_workspace_bytes(g->B, g->V, g->top_n))
       return set_error(ARCS_ERR_WORKSPACE, "logprobs_batch: workspace too small");
     if ((reinterpret_cast<uintptr_t>(g->workspace) & 15u) != 0) return set_error(ARCS_ERR_WORKSPACE, "logprobs_batch: workspace must be 16-byte aligned");
@@ -515,17 +655,15 @@ extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
     a.ws_ctr = reinterpret_cast<unsigned int*>(ws);
     ws += ((size_t)g->B * 4 + 255) & ~(size_t)255;
     a.ws_part = reinterpret_cast<LpPart*>(ws);
-    ws += (size_t)g->B * a.nseg * sizeof(LpPart);
+    ws += (size_t)g->B * a.max_pieces * sizeof(LpPart);
     a.ws_list = reinterpret_cast<unsigned long long*>(ws);
   }
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const unsigned grid = (unsigned)g->B * (unsigned)a.nseg;
-#define ARCS_LAUNCH(T)                                                                                               \
-  do {                                                                                                               \
-    static std::atomic<unsigned long long> attr_done{0};                                                   \
-    cudaError_t e = ensure_dynamic_smem(logprob_kernel<T>, (int)kLpSmem, attr_done);                       \
-    if (e != cudaSuccess) return set_error(ARCS_ERR_CUDA, cudaGetErrorString(e));                                    \
-    logprob_kernel<T><<<grid, kThreads, kLpSmem, st>>>(a);                                                           \
+#define ARCS_LAUNCH(T)                                                                            \
+  do {                                                                                            \
+    if (g->top_n == 0) logprob_kernel<T, 0><<<plan.grid, kLpThreads, 0, st>>>(a);                   \
+    else if (g->top_n <= kLpFew) logprob_kernel<T, 1><<<plan.grid, kLpThreads, 0, st>>>(a);         \
+    else logprob_kernel<T, 2><<<plan.grid, kLpThreads, 0, st>>>(a);                                 \
   } while (0)
   if (g->dtype == ARCS_F32) ARCS_LAUNCH(float);
   else ARCS_LAUNCH(__nv_bfloat16);

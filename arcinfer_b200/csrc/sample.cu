@@ -3,8 +3,11 @@
 // prepares each item's touched tokens ahead of the pass) and finish (per row: order, softmax,
 // cuts, draw), which runs beside the stream kernel and takes each row as it is released. The
 // kernels hand their results on through the workspace.
+#include <algorithm>
+
 #include "sample_finish.cuh"
 #include "sample_stream.cuh"
+#include "sample_resident.cuh"
 
 using namespace arcs;
 
@@ -27,6 +30,8 @@ static cudaError_t launch_dependent(K kernel, unsigned grid, unsigned block, siz
 
 constexpr int kMaxRows = 65536;
 constexpr int kItemsPerSm = 1;        // work items per SM that few rows are cut into
+constexpr size_t kResSmemMax = 227 * 1024;
+constexpr int kResWaves = 1;
 constexpr int kFinishThreads = 128;   // threads of the finish kernel's CTA (four rows per CTA; one with an allowed-token mask)
 
 // Rows with an allowed-token mask are not cut: the ranked head needs the 512 best of the whole
@@ -52,6 +57,49 @@ extern "C" size_t arcs_sample_workspace_bytes(int32_t B, int32_t V, int32_t mask
   int nseg, seg_len;
   plan_items(B, V, masked != 0, &nseg, &seg_len);
   return (size_t)B * nseg * (size_t)item_block_bytes(masked != 0, table_slots(max_list));
+}
+
+// Which rows are held on the chip (sample_resident.cuh): RULE_COMMENT
+struct ResPlan {
+  int ctas = 0;       // CTAs (of one cluster) a row, 0: not taken
+  int slice = 0;      // columns a CTA holds
+  size_t smem = 0;
+};
+static ResPlan plan_resident(int B, int V, int elt, int max_hist, int max_bias) {
+  ResPlan p;
+  if (max_hist + max_bias > kResMaxList) return p;
+  const size_t fixed = ((sizeof(ResShared) + 15) & ~(size_t)15) + res_list_bytes(max_hist, max_bias) + 128;
+  for (int c = 1; c <= 8; c *= 2) {
+    const int64_t slice = ((int64_t)V + c * 64 - 1) / (c * 64) * 64;
+    const size_t smem = fixed + (size_t)slice * elt;
+    if (smem > kResSmemMax) continue;
+    if (p.ctas != 0 && (int64_t)B * c > kSmCount) break;  // (more CTAs a row only while they are at work at once)
+    if (c > 1 && p.ctas != 0 && slice * elt < 16384) break;
+    p.ctas = c;
+    p.slice = (int)slice;
+    p.smem = smem;
+  }
+  const int64_t per_sm = p.ctas ? std::max<int64_t>(1, (int64_t)(228 * 1024) / (int64_t)(p.smem + 1024)) : 1;
+  if (p.ctas && (int64_t)B * p.ctas > kResWaves * kSmCount * std::min<int64_t>(per_sm, 2)) p.ctas = 0;
+  return p;
+}
+template <typename T>
+static cudaError_t launch_resident(const SampleDev& a, const ResPlan& p, cudaStream_t st) {
+  static std::atomic<unsigned long long> attr_done{0};
+  cudaError_t e = ensure_dynamic_smem(resident_kernel<T>, (int)kResSmemMax, attr_done);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(a.B * p.ctas));
+  cfg.blockDim = dim3(kResThreads);
+  cfg.dynamicSmemBytes = p.smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)p.ctas;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, resident_kernel<T>, a, p.ctas, p.slice);
 }
 
 // events[0..2], when given, are recorded before the first launch and after each of the two
@@ -131,8 +179,18 @@ static int sample_launch(const arcs_sample_args* g, void* stream, cudaEvent_t* e
     return set_error(ARCS_ERR_WORKSPACE, "sample_batch: workspace too small");
   if ((reinterpret_cast<uintptr_t>(g->workspace) & 15u) != 0) return set_error(ARCS_ERR_WORKSPACE, "sample_batch: workspace must be 16-byte aligned");
 
-  const size_t smem_s = stream_smem_bytes(masked, slots);
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (!masked) {
+    const ResPlan rp = plan_resident(a.B, a.V, g->dtype == ARCS_F32 ? 4 : 2, a.max_hist, a.max_bias);
+    if (rp.ctas > 0) {
+      if (events) cudaEventRecord(events[0], st);
+      const cudaError_t e = g->dtype == ARCS_F32 ? launch_resident<float>(a, rp, st) : launch_resident<__nv_bfloat16>(a, rp, st);
+      if (e != cudaSuccess) return set_error(ARCS_ERR_CUDA, cudaGetErrorString(e));
+      for (int i = 1; events && i < 3; ++i) cudaEventRecord(events[i], st);
+      return check_launch("sample_batch");
+    }
+  }
+  const size_t smem_s = stream_smem_bytes(masked, slots);
   const int items = a.nseg * a.B;
   const unsigned grid_s = (unsigned)(items < kSmCount ? items : kSmCount);
 #define ARCS_LAUNCH(T, M)                                                                                          \

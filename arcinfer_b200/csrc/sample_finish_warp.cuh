@@ -102,6 +102,89 @@ __device__ __forceinline__ void combine_mz(const SampleDev& a, int b) {
   }
 }
 
+// tools/sampler.h:54-77 for row b by one warp: from its nB candidates best first (values sv, ids sid)
+// to the token and the other outputs. spr, cum: nB doubles of scratch each; bans: the row's bias list
+// bans some token.
+__device__ __forceinline__ void choose_token(const SampleDev& a, int b, const RowCfg& r, bool bans, int nB, const float* sv, const int32_t* sid,
+                                             double* spr, double* cum) {
+  const int lane = threadIdx.x & 31;
+  int nc = nB;
+  if (bans)  // :54-55 (every lane walks the same few steps)
+    while (nc > 1 && sv[nc - 1] <= ARCS_BANNED) --nc;
+  bool tie = false;  // equal logits among the candidates kept: the reference's order there is not defined
+  for (int i = lane; i + 1 < nc; i += 32) tie = tie || sv[i] == sv[i + 1];
+  const int flags = __any_sync(0xFFFFFFFFu, tie) ? ARCS_FLAG_TIE_TOPK : 0;
+  const bool draw = !r.greedy && nc >= 1;
+  int token = nc > 0 ? sid[0] : -1, n = nc > 0 ? 1 : 0;
+  if (draw) {
+    const float mx = sv[0];
+    for (int i = lane; i < nc; i += 32) {
+      const float x = __fdiv_rn(__fsub_rn(sv[i], mx), r.prm.temperature);  // :60 float arithmetic
+      spr[i] = (double)exp_term(x);                                        // float exp, widened
+    }
+    __syncwarp();
+    double z = 0.0;  // :58-60 in candidate order (every lane adds the same chain)
+#pragma unroll 8
+    for (int i = 0; i < nc; ++i) z = __dadd_rn(z, spr[i]);
+    __syncwarp();
+    for (int i = lane; i < nc; i += 32) spr[i] = __ddiv_rn(spr[i], z);  // :64, the same quotients in any order
+    __syncwarp();
+    // :65-72. The running sums are a chain of roundings in candidate order; where the chain is
+    // cut is then found by all lanes.
+    if (lane == 0) {
+      double c = 0.0;
+#pragma unroll 8
+      for (int i = 0; i < nc; ++i) {
+        c = __dadd_rn(c, spr[i]);
+        cum[i] = c;
+      }
+    }
+    __syncwarp();
+    const double mp = __dmul_rn((double)r.prm.min_p, spr[0]);
+    int n_i = nc;
+    for (int i = lane; i < nc; i += 32) {
+      int c = 0x7FFFFFFF;
+      if (r.prm.min_p > 0.0f && spr[i] < mp) c = max(1, i);   // :65 (tested before the candidate is added)
+      else if (cum[i] >= (double)r.prm.top_p) c = i + 1;         // :67
+      n_i = min(n_i, c);
+    }
+    n = (int)__reduce_min_sync(0xFFFFFFFFu, (unsigned)n_i);
+    if (lane == 0) {
+      const double tot = cum[n - 1];             // the same sum, in the same order, as :70
+      double rr = __dmul_rn(a.u[b], tot);        // :71-72
+      int pick = -1;
+      for (int i = 0; i < n && pick < 0; i += 4) {  // (four steps of the chain at a time: the loads run ahead of it)
+        const double p0 = spr[i], p1 = i + 1 < n ? spr[i + 1] : 0.0, p2 = i + 2 < n ? spr[i + 2] : 0.0, p3 = i + 3 < n ? spr[i + 3] : 0.0;
+        const double r0 = __dsub_rn(rr, p0), r1 = __dsub_rn(r0, p1), r2 = __dsub_rn(r1, p2), r3 = __dsub_rn(r2, p3);
+        if (r0 <= 0.0) pick = i;
+        else if (i + 1 < n && r1 <= 0.0) pick = i + 1;
+        else if (i + 2 < n && r2 <= 0.0) pick = i + 2;
+        else if (i + 3 < n && r3 <= 0.0) pick = i + 3;
+        rr = r3;
+      }
+      if (pick < 0) pick = n - 1;
+      token = sid[pick];
+    }
+  }
+  if (lane == 0) {
+    if (r.k_bad || !r.lists_ok) token = -1;
+    a.token[b] = token;
+    if (a.n_cand) a.n_cand[b] = nc;
+    if (a.n_kept) a.n_kept[b] = n;
+    if (a.flags) a.flags[b] = flags;
+  }
+  if (a.cand_id || a.cand_val || a.cand_pr) {
+    if (lane == 0 && nc > a.cand_width) raise_status(a.status, ARCS_ERR_TOPK);
+    for (int i = lane; i < a.cand_width; i += 32) {
+      const size_t o = (size_t)b * a.cand_stride + i;
+      const bool in = i < nc;
+      if (a.cand_id) a.cand_id[o] = in ? sid[i] : -1;
+      if (a.cand_val) a.cand_val[o] = in ? sv[i] : 0.0f;
+      if (a.cand_pr) a.cand_pr[o] = in ? (draw ? (float)spr[i] : (i == 0 ? 1.0f : 0.0f)) : 0.0f;
+    }
+  }
+}
+
 // NT threads finish row b: one warp (NT == 32, four rows to a CTA), or the whole CTA (NT == 128)
 // when the rows are few, which are then cut into many segments with as many loose thresholds:
 // the entries are read by all threads, the threshold is tightened from a count of the entries by
@@ -409,83 +492,7 @@ __device__ __noinline__ int finish_row_fast(const SampleDev& a, int b, FastScrat
   else rank_all(IntTag<kFastBuf / 32>{});
   bar();
   if (!lead) return kFastDone;  // (the rest is one warp's work)
-  // ---- tools/sampler.h:54-77
-  int nc = nB;
-  if (bans)  // :54-55 (every lane walks the same few steps)
-    while (nc > 1 && fs.sv[nc - 1] <= ARCS_BANNED) --nc;
-  bool tie = false;  // equal logits among the candidates kept: the reference's order there is not defined
-  for (int i = lane; i + 1 < nc; i += 32) tie = tie || fs.sv[i] == fs.sv[i + 1];
-  const int flags = __any_sync(0xFFFFFFFFu, tie) ? ARCS_FLAG_TIE_TOPK : 0;
-  const bool draw = !r.greedy && nc >= 1;
-  int token = nc > 0 ? fs.sid[0] : -1, n = nc > 0 ? 1 : 0;
-  double* cum = reinterpret_cast<double*>(fs.buf);  // (the buffer is no longer needed)
-  if (draw) {
-    const float mx = fs.sv[0];
-    for (int i = lane; i < nc; i += 32) {
-      const float x = __fdiv_rn(__fsub_rn(fs.sv[i], mx), r.prm.temperature);  // :60 float arithmetic
-      fs.spr[i] = (double)exp_term(x);                                        // float exp, widened
-    }
-    __syncwarp();
-    double z = 0.0;  // :58-60 in candidate order (every lane adds the same chain)
-#pragma unroll 8
-    for (int i = 0; i < nc; ++i) z = __dadd_rn(z, fs.spr[i]);
-    __syncwarp();
-    for (int i = lane; i < nc; i += 32) fs.spr[i] = __ddiv_rn(fs.spr[i], z);  // :64, the same quotients in any order
-    __syncwarp();
-    // :65-72. The running sums are a chain of roundings in candidate order; where the chain is
-    // cut is then found by all lanes.
-    if (lane == 0) {
-      double c = 0.0;
-#pragma unroll 8
-      for (int i = 0; i < nc; ++i) {
-        c = __dadd_rn(c, fs.spr[i]);
-        cum[i] = c;
-      }
-    }
-    __syncwarp();
-    const double mp = __dmul_rn((double)r.prm.min_p, fs.spr[0]);
-    int n_i = nc;
-    for (int i = lane; i < nc; i += 32) {
-      int c = 0x7FFFFFFF;
-      if (r.prm.min_p > 0.0f && fs.spr[i] < mp) c = max(1, i);   // :65 (tested before the candidate is added)
-      else if (cum[i] >= (double)r.prm.top_p) c = i + 1;         // :67
-      n_i = min(n_i, c);
-    }
-    n = (int)__reduce_min_sync(0xFFFFFFFFu, (unsigned)n_i);
-    if (lane == 0) {
-      const double tot = cum[n - 1];             // the same sum, in the same order, as :70
-      double rr = __dmul_rn(a.u[b], tot);        // :71-72
-      int pick = -1;
-      for (int i = 0; i < n && pick < 0; i += 4) {  // (four steps of the chain at a time: the loads run ahead of it)
-        const double p0 = fs.spr[i], p1 = i + 1 < n ? fs.spr[i + 1] : 0.0, p2 = i + 2 < n ? fs.spr[i + 2] : 0.0, p3 = i + 3 < n ? fs.spr[i + 3] : 0.0;
-        const double r0 = __dsub_rn(rr, p0), r1 = __dsub_rn(r0, p1), r2 = __dsub_rn(r1, p2), r3 = __dsub_rn(r2, p3);
-        if (r0 <= 0.0) pick = i;
-        else if (i + 1 < n && r1 <= 0.0) pick = i + 1;
-        else if (i + 2 < n && r2 <= 0.0) pick = i + 2;
-        else if (i + 3 < n && r3 <= 0.0) pick = i + 3;
-        rr = r3;
-      }
-      if (pick < 0) pick = n - 1;
-      token = fs.sid[pick];
-    }
-  }
-  if (lane == 0) {
-    if (r.k_bad || !r.lists_ok) token = -1;
-    a.token[b] = token;
-    if (a.n_cand) a.n_cand[b] = nc;
-    if (a.n_kept) a.n_kept[b] = n;
-    if (a.flags) a.flags[b] = flags;
-  }
-  if (a.cand_id || a.cand_val || a.cand_pr) {
-    if (lane == 0 && nc > a.cand_width) raise_status(a.status, ARCS_ERR_TOPK);
-    for (int i = lane; i < a.cand_width; i += 32) {
-      const size_t o = (size_t)b * a.cand_stride + i;
-      const bool in = i < nc;
-      if (a.cand_id) a.cand_id[o] = in ? fs.sid[i] : -1;
-      if (a.cand_val) a.cand_val[o] = in ? fs.sv[i] : 0.0f;
-      if (a.cand_pr) a.cand_pr[o] = in ? (draw ? (float)fs.spr[i] : (i == 0 ? 1.0f : 0.0f)) : 0.0f;
-    }
-  }
+  choose_token(a, b, r, bans, nB, fs.sv, fs.sid, fs.spr, reinterpret_cast<double*>(fs.buf));  // (the buffer is no longer needed)
   return kFastDone;
 }
 

@@ -176,6 +176,49 @@ __device__ __noinline__ void sel_prune(const Sel& s, int k, const PruneScratch& 
   group_sync<BAR, G>();
 }
 
+// Warp-collective append to the candidate buffer; lanes with p set store (key, id). Returns true
+// for a lane whose entry found no room (the caller offers it again after the next prune); `hot`
+// is set once the buffer has grown past the prune trigger.
+__device__ __forceinline__ bool sel_offer(const Sel& s, bool p, uint32_t key, int32_t id, bool& hot) {
+  const unsigned b = __ballot_sync(0xFFFFFFFFu, p);
+  if (b == 0) return false;
+  const int lane = threadIdx.x & 31, leader = __ffs(b) - 1;
+  int base = 0;
+  if (lane == leader) base = (int)sm_atomic_add(s.cnt, (uint32_t)__popc(b));
+  base = __shfl_sync(0xFFFFFFFFu, base, leader);
+  if (!p) return false;
+  const int pos = base + __popc(b & ((1u << lane) - 1u));
+  hot = hot || pos + 1 > s.trig;
+  if (pos >= s.cap) return true;
+  s.key[pos] = key;
+  s.id[pos] = id;
+  return false;
+}
+// Every thread calls with the mask of its own elements that may belong to the n best;
+// elem(idx, key, id) names element idx. When the buffer has grown past the trigger, or had no room
+// for some entry, the CTA keeps the n best, the threshold rises and what was left out is offered
+// again. The buffer's count and threshold are quiescent on entry and on return.
+template <int NT, typename ELEM>
+__device__ __forceinline__ void push_all(const Sel& sel, const PruneScratch& ps, uint32_t bits, ELEM elem) {
+  for (;;) {
+    uint32_t again = 0;
+    bool hot = false;
+    const unsigned long long tau = *sel.tau;
+    while (__any_sync(0xFFFFFFFFu, bits != 0u)) {
+      uint32_t ky = 0;
+      int32_t id = 0;
+      const int idx = bits != 0u ? __ffs(bits) - 1 : 0;
+      if (bits != 0u) elem(idx, ky, id);
+      const bool p = bits != 0u && ky != 0u && comp_of(ky, id) > tau;
+      bits &= bits - 1u;
+      if (sel_offer(sel, p, ky, id, hot)) again |= 1u << idx;
+    }
+    if (!__syncthreads_or(hot || again != 0u)) break;
+    sel_prune<1, NT>(sel, sel.k, ps, threadIdx.x);
+    __syncthreads();
+    bits = again;
+  }
+}
 
 // A lower bound of the kth largest (1-based) of 32 * PER keys held PER to a lane, found by ONE
 // warp with a search on the keys' upper 16 bits, two bits a round (bf16 resolution; exact for

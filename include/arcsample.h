@@ -307,13 +307,13 @@ void arcs_jcon_destroy(arcs_jcon* h);
  * logprobs_batch: per row, the log probability of one token and the top_n most likely
  * alternatives, from the RAW logits (no penalty, no bias): the `logprobs` entry of
  * tools/server_chat.h:417-441, and the log-softmax that scores perplexity and KL
- * (zero/runz.cpp:478-484, :639-646). One pass over the logits, one launch. When there are few
- * rows each is cut into segments, whose results meet in the workspace.
+ * (zero/runz.cpp:478-484, :639-646). One pass over the logits, one launch. The rows are dealt out
+ * evenly to the SMs; where a row is cut, its pieces' results meet in the workspace.
  *   mx = max; z = sum exp(l - mx) accumulated in fp64; lse = mx + log(z);
  *   logprob[b] = l[token[b]] - lse;  top_id / top_logprob: the top_n largest logits, best first
  *   (equal logits: lower id first), as log probabilities.
  * The reference sums fp64 exponentials in index order; here each term is a single-precision
- * exponential (ex2.approx of the rounded product (l - m) * log2 e), summed pairwise in fp32 per
+ * exponential (ex2.approx of the product (l - m) * log2 e rounded once), summed pairwise in fp32 per
  * 16-byte chunk and then in fp64, in another order: lse agrees with an fp64 log-sum-exp to about
  * 4e-8 absolute on the tested distributions (the tests hold it to 1e-6). NaN logits are skipped.
  * ---------------------------------------------------------------------------------------- */
