@@ -1,5 +1,5 @@
 // sample_batch: penalties + temperature / top-k / top-p / min-p (+ allowed-token mask) with one
-// pass over the logits. Two launches on the caller's stream: stream (the pass itself, which also
+// pass over the logits. Rows that fit on the chip: one launch (sample_resident.cuh). Others: two launches on the caller's stream: stream (the pass itself, which also
 // prepares each item's touched tokens ahead of the pass) and finish (per row: order, softmax,
 // cuts, draw), which runs beside the stream kernel and takes each row as it is released. The
 // kernels hand their results on through the workspace.
@@ -31,7 +31,6 @@ static cudaError_t launch_dependent(K kernel, unsigned grid, unsigned block, siz
 constexpr int kMaxRows = 65536;
 constexpr int kItemsPerSm = 1;        // work items per SM that few rows are cut into
 constexpr size_t kResSmemMax = 227 * 1024;
-constexpr int kResWaves = 1;
 constexpr int kFinishThreads = 128;   // threads of the finish kernel's CTA (four rows per CTA; one with an allowed-token mask)
 
 // Rows with an allowed-token mask are not cut: the ranked head needs the 512 best of the whole
@@ -59,7 +58,13 @@ extern "C" size_t arcs_sample_workspace_bytes(int32_t B, int32_t V, int32_t mask
   return (size_t)B * nseg * (size_t)item_block_bytes(masked != 0, table_slots(max_list));
 }
 
-// Which rows are held on the chip (sample_resident.cuh): RULE_COMMENT
+// Which rows are held on the chip (sample_resident.cuh): those of a call whose CTAs, each with as
+// large a slice as fits its SM's shared memory, are at work all at once or one and a half times
+// over. Measured (history 256, top-k 50; stream + finish kernel -> resident): 1 x 151936 fp32
+// 37 -> 20 us a call, 32 x 151936 fp32 (128 CTAs) 45 -> 21, 48 (192 CTAs) 45 -> 35, 64 (256 CTAs)
+// 45 -> 39, 74 (296 CTAs) 41 -> 49; 74 x 151936 bf16 (148 CTAs) 38 -> 23, 96 (192) 40 -> 39;
+// 16 x 262144 fp32 (128 CTAs) 45 -> 33; 296 x 32000 bf16 (two CTAs an SM) 37 -> 23, 400: 40 -> 41.
+// A row takes more CTAs, up to a portable cluster's eight, only while no SM then has to take two.
 struct ResPlan {
   int ctas = 0;       // CTAs (of one cluster) a row, 0: not taken
   int slice = 0;      // columns a CTA holds
@@ -80,7 +85,7 @@ static ResPlan plan_resident(int B, int V, int elt, int max_hist, int max_bias) 
     p.smem = smem;
   }
   const int64_t per_sm = p.ctas ? std::max<int64_t>(1, (int64_t)(228 * 1024) / (int64_t)(p.smem + 1024)) : 1;
-  if (p.ctas && (int64_t)B * p.ctas > kResWaves * kSmCount * std::min<int64_t>(per_sm, 2)) p.ctas = 0;
+  if (p.ctas && (int64_t)B * p.ctas * 2 > 3 * kSmCount * std::min<int64_t>(per_sm, 2)) p.ctas = 0;
   return p;
 }
 template <typename T>

@@ -11,7 +11,10 @@
 //     reaches it, and the adjusted columns that do, are the slice's candidates (a few more than k);
 //  4. the cluster's first CTA reads the others' candidates out of their shared memory, ranks them
 //     and follows tools/sampler.h:54-77.
-// What bounds it: latency. RES_MEASURED
+// What bounds it: latency, spread over all steps. 1 x 151936 fp32, history 64 (8 CTAs of 76 KB), in us
+// from the CTA's start: lists 0.7, slice there 2.0, maxima 2.9, threshold 4.0, candidates 5.8, cluster
+// barrier 7.7, fetched and cut 9.6, ranked 10.6, token 12.9; a call 31 -> 15 us. 8 x 262144 fp32
+// 45 -> 22 us, 64 x 151936 bf16 (two CTAs of 152 KB a row) about 38 -> 23 us.
 #pragma once
 #include "sample_finish_warp.cuh"
 
@@ -41,8 +44,9 @@ struct ResShared {
   uint32_t scal[16];                        // the elements before and after the aligned body, as float bits
 };
 
-// history entries of the slice (column, place), the row's bias list, the adjusted columns (key, id)
-__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)max_hist * 8 + (size_t)max_bias * 8 + (size_t)(max_hist + max_bias) * 8; }
+// history entries of the slice (column, place: padded to four), the row's bias list, what applies to
+// the columns, the adjusted columns (key, id)
+__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)(max_hist + 4) * 8 + (size_t)max_bias * 8 + (size_t)(max_hist + max_bias) * 12; }
 
 __device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
   uint32_t r;
@@ -69,10 +73,11 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   constexpr int E = Elem<T>::kPerChunk;
   constexpr int NT = kResThreads;
   int32_t* const h_col = reinterpret_cast<int32_t*>(res_smem + ((sizeof(ResShared) + 15) & ~(size_t)15));
-  int32_t* const h_at = h_col + a.max_hist;
-  int32_t* const b_id = h_at + a.max_hist;
+  int32_t* const h_at = h_col + a.max_hist + 4;
+  int32_t* const b_id = h_at + a.max_hist + 4;
   float* const b_val = reinterpret_cast<float*>(b_id + a.max_bias);
-  uint32_t* const t_key = reinterpret_cast<uint32_t*>(b_val + a.max_bias);
+  uint32_t* const info = reinterpret_cast<uint32_t*>(b_val + a.max_bias);
+  uint32_t* const t_key = info + a.max_hist + a.max_bias;
   int32_t* const t_id = reinterpret_cast<int32_t*>(t_key + a.max_hist + a.max_bias);
   char* const data = res_smem + (((size_t)(reinterpret_cast<char*>(t_id + a.max_hist + a.max_bias) - res_smem) + 127) & ~(size_t)127);
 
@@ -82,7 +87,8 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   const int32_t lo = min(a.V, rank * slice), hi = min(a.V, lo + slice);
   const SegPlan p = make_plan(row, lo, hi);
   const int nchunk = p.body_bytes / 16;
-  const int part = ((nchunk + kResParts - 1) / kResParts + NT - 1) / NT * NT;  // chunks a copy brings
+  constexpr int kRound = kResOwn * NT;  // chunks the threads look at together: chunk c is thread c % NT's, its maximum number c / NT % kResOwn
+  const int part = ((nchunk + kResParts - 1) / kResParts + kRound - 1) / kRound * kRound;  // chunks a copy brings
   if (tid == 0) {
     for (int i = 0; i < kResParts; ++i) mbar_init(&s.bars[i], 1);
     mbar_init_fence();
@@ -131,11 +137,52 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
     if (i * part < nchunk) ok = ok && mbar_wait_warp(&s.bars[i], 0u);
   };
   if (lists) {
-    for (int i = 0; i < kResParts; ++i) wait_part(i);
     const int L = s.n_hist;
     const int32_t w0 = window_start(r);
+    if (tid < 4) h_col[L + tid] = -1;
+    __syncthreads();
+    // What applies to a column, while the slice is on its way: its occurrences in the history, whether
+    // one lies in the repeat window (bit 31), and whether the entry at place `at` is its first (else 0).
+    auto occurrences = [&](int32_t c, int32_t at, bool& first) -> uint32_t {
+      uint32_t cnt = 0, win = 0;
+#pragma unroll 4
+      for (int j = 0; j < L; j += 4) {
+        const int4 q = *reinterpret_cast<const int4*>(&h_col[j]);
+        if (q.x == c || q.y == c || q.z == c || q.w == c) {
+          const int32_t e[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int x = 0; x < 4; ++x)
+            if (e[x] == c) {
+              ++cnt;
+              if (h_at[j + x] >= w0) win = 1u << 31;
+              first = first && h_at[j + x] >= at;
+            }
+        }
+      }
+      return cnt | win;
+    };
+    // (a column is taken by its first bias entry, or, without one, by its first history entry)
+    constexpr uint32_t kTake = 1u << 30;
+    for (int i = tid; i < NB; i += NT) {
+      const int32_t c = b_id[i] - a.id_base;
+      bool first = b_id[i] >= 0 && c >= lo && c < hi, none = true;
+      for (int j = 0; j < i && first; ++j) first = b_id[j] != b_id[i];
+      info[i] = first ? kTake | occurrences(c, -1, none) : 0u;
+    }
+    for (int i = tid; i < L; i += NT) {
+      const int32_t c = h_col[i];
+      bool first = true;
+      for (int j = 0; j < NB && first; ++j) first = b_id[j] != c + a.id_base;
+      const uint32_t o = first ? occurrences(c, h_at[i], first) : 0u;
+      info[NB + i] = first ? kTake | o : 0u;
+    }
+    __syncthreads();
+    for (int i = 0; i < kResParts; ++i) wait_part(i);
     // one column adjusted (tools/sampler.h:154-174): the raw logit from the slice, a NaN into its place
-    auto adjust = [&](int32_t c, bool biased, int first_bias) {
+    for (int i = tid; i < NB + L; i += NT) {
+      const uint32_t o = info[i];
+      if (!(o & kTake)) continue;
+      const int32_t c = i < NB ? b_id[i] - a.id_base : h_col[i - NB];
       float v;
       if (c >= p.body_first && c < p.tail_first) {
         T* at = reinterpret_cast<T*>(data) + (c - p.body_first);
@@ -148,40 +195,17 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
         *at = 0x7FFFFFFFu;
       }
       bool ban = false;
-      if (biased) {
-        const int32_t t = c + a.id_base;
-        for (int j = first_bias; j < NB; ++j) {  // :154-155 in list order, duplicates add again
-          if (b_id[j] != t) continue;
-          if (b_val[j] > -100.0f) v = __fadd_rn(v, b_val[j]);
-          else ban = true;
-        }
+      for (int j = i; j < NB; ++j) {  // :154-155 in list order, duplicates add again
+        if (b_id[j] != c + a.id_base) continue;
+        if (b_val[j] > -100.0f) v = __fadd_rn(v, b_val[j]);
+        else ban = true;
       }
-      uint32_t cnt = 0;
-      bool win = false;
-      for (int j = 0; j < L; ++j)
-        if (h_col[j] == c) {
-          ++cnt;
-          win = win || h_at[j] >= w0;
-        }
-      if (cnt > 0) v = penalise(r, v, cnt, win);
+      const uint32_t cnt = o & (kTake - 1u);
+      if (cnt > 0) v = penalise(r, v, cnt, (o >> 31) != 0u);
       if (ban) v = ARCS_BANNED;                                                                        // :174
       const int at = (int)sm_atomic_add(&s.n_touch, 1u);
       t_key[at] = key_of(v);
       t_id[at] = c + a.id_base;
-    };
-    // (a column is taken by its first bias entry, or, without one, by its first history entry)
-    for (int i = tid; i < NB; i += NT) {
-      const int32_t c = b_id[i] - a.id_base;
-      bool first = b_id[i] >= 0 && c >= lo && c < hi;
-      for (int j = 0; j < i && first; ++j) first = b_id[j] != b_id[i];
-      if (first) adjust(c, true, i);
-    }
-    for (int i = tid; i < L; i += NT) {
-      const int32_t c = h_col[i], at = h_at[i];
-      bool first = true;
-      for (int j = 0; j < NB && first; ++j) first = b_id[j] != c + a.id_base;
-      for (int j = 0; j < L && first; ++j) first = h_col[j] != c || h_at[j] >= at;
-      if (first) adjust(c, false, 0);
     }
     __syncthreads();
   }
@@ -193,7 +217,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   for (int i = 0; i < kResParts; ++i) {
     wait_part(i);
     const int end = min(nchunk, (i + 1) * part);
-    for (int c0 = i * part + tid; c0 < end; c0 += kResOwn * NT) {
+    for (int c0 = i * part + tid; c0 < end; c0 += kRound) {
 #pragma unroll
       for (int j = 0; j < kResOwn; ++j)
         if (c0 + j * NT < end) own[j] = fmaxf(own[j], Elem<T>::chunk_max(lds128(data + (size_t)(c0 + j * NT) * 16)));
@@ -235,18 +259,22 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
         s.id[at] = id;
       }
     };
+    // the chunks behind a maximum that reaches it, looked through by the whole warp
 #pragma unroll
     for (int j = 0; j < kResOwn; ++j) {
-      if (!(own[j] >= tf) || s.failed) continue;
-      for (int i = 0; i < kResParts; ++i) {
-        const int end = min(nchunk, (i + 1) * part);
-        for (int c = i * part + j * NT + tid; c < end; c += kResOwn * NT) {
+      unsigned hot = __ballot_sync(0xFFFFFFFFu, own[j] >= tf && !s.failed);
+      while (hot != 0u) {
+        const int src = (tid & ~31) + __ffs(hot) - 1;
+        hot &= hot - 1u;
+        for (int c = j * NT + src + lane * kRound; c < nchunk; c += 32 * kRound) {
           const uint4 q = lds128(data + (size_t)c * 16);
-          if (!(Elem<T>::chunk_max(q) >= tf)) continue;
+          uint32_t bits = 0;
 #pragma unroll
-          for (int e = 0; e < E; ++e) {
-            const float v = Elem<T>::get(q, e);
-            if (v >= tf) keep(key_of(v), p.body_first + c * E + e + a.id_base);
+          for (int e = 0; e < E; ++e) bits |= (Elem<T>::get(q, e) >= tf ? 1u : 0u) << e;
+          while (bits != 0u) {
+            const int e = __ffs(bits) - 1;
+            bits &= bits - 1u;
+            keep(key_of(elem_of_words<T>(q.x, q.y, q.z, q.w, e)), p.body_first + c * E + e + a.id_base);
           }
         }
       }
@@ -318,24 +346,46 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       s.mcnt = 0;
       s.misc[4] = any_bad;
     }
+  } else {
+    for (int i = tid - 32; i < 256; i += NT - 32) s.keys[i] = 0u;
   }
   __syncthreads();
   const int total = s.off[ctas];
-  if (total <= 4 * NT) {  // (as a rule: fetched in one go)
-    for (int e0 = 0; e0 < total; e0 += NT) {
-      const int e = e0 + tid;
-      int g = 0;
-      for (int x = 1; x < ctas; ++x) g += e >= s.off[x];
-      const bool have = e < total;
-      uint32_t k0 = 0;
-      int32_t i0 = 0;
-      if (have) {
-        k0 = cluster_ld(&s.key[e - s.off[g]], g);
-        i0 = (int32_t)cluster_ld(&s.id[e - s.off[g]], g);
+  if (total <= 4 * NT) {
+    // As a rule: fetched in one go, and a tighter threshold read off their counts by the upper 16 bits
+    // of their keys, before they are kept.
+    uint32_t k0[4];
+    int32_t i0[4];
+    const uint32_t base = (uint32_t)(s.tau >> 48);
+    const unsigned long long tau0 = s.tau;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int e = x * NT + tid;
+      k0[x] = 0u;
+      i0[x] = 0;
+      if (e < total) {
+        int g = 0;
+        for (int y = 1; y < ctas; ++y) g += e >= s.off[y];
+        k0[x] = cluster_ld(&s.key[e - s.off[g]], g);
+        i0[x] = (int32_t)cluster_ld(&s.id[e - s.off[g]], g);
       }
-      bool hot = false;
-      sel_offer(sel, have && comp_of(k0, i0) > s.tau, k0, i0, hot);
     }
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (k0[x] != 0u && comp_of(k0[x], i0[x]) > tau0) sm_red_add(&s.keys[min((k0[x] >> 16) - base, 255u)], 1u);
+    __syncthreads();
+    if (tid < 32) {
+      int d, kr;
+      bool ex;
+      find_bin(s.keys, kB, d, kr, ex);
+      if (d > 0 && lane == 0) s.tau = max(tau0, ((unsigned long long)((base + (uint32_t)d) << 16) << 32) - 1ull);
+    }
+    __syncthreads();
+    bool hot = false;
+    const unsigned long long tau1 = s.tau;
+#pragma unroll
+    for (int x = 0; x < 4; ++x)
+      if (x * NT < total) sel_offer(sel, k0[x] != 0u && comp_of(k0[x], i0[x]) > tau1, k0[x], i0[x], hot);
   } else {
     for (int e0 = 0; e0 < total; e0 += NT) {
       const int e = e0 + tid;

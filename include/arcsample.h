@@ -62,8 +62,8 @@ const char* arcs_last_error(void); /* text of the calling thread's last failure 
 int arcs_version(void);
 
 /* ------------------------------------------------------------------------------------------
- * sample_batch: Sampler::adjusted + Sampler::sample for B rows in one call (two launches on the
- * stream: the single pass over the logits, and a small per-row finish that runs beside it)
+ * sample_batch: Sampler::adjusted + Sampler::sample for B rows in one call (one launch while the rows
+ * fit on the chip; else two: the single pass over the logits, and a small per-row finish beside it)
  * (tools/sampler.h:36-78, :147-176); with a mask, Sampler::sample_allowed (:82-144) where
  * the predicate ok(t) is bit t of the row's mask.
  * ---------------------------------------------------------------------------------------- */
@@ -121,9 +121,10 @@ typedef struct {
 /* max_list: max_hist + max_bias of the call (0 without lists) */
 size_t arcs_sample_workspace_bytes(int32_t B, int32_t V, int32_t masked, int32_t max_list);
 int arcs_sample_batch(const arcs_sample_args* args, void* stream);
-/* Measurement aid: the same two launches, one after the other (the finish kernel does not run
+/* Measurement aid: the same launches, one after the other (the finish kernel does not run
  * beside the stream kernel here), with CUDA events between them on `stream`; waits for them and
- * returns the device time of the stream and finish kernels in ms2[0..1]. */
+ * returns the device time of the stream and finish kernels in ms2[0..1] (of the one kernel, and
+ * nothing, where the rows are held on the chip). */
 int arcs_sample_batch_timed(const arcs_sample_args* args, void* stream, float* ms2);
 
 /* adjusted_batch: Sampler::adjusted (tools/sampler.h:147-176) for whole rows: the logits after
