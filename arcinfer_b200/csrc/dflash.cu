@@ -4,8 +4,11 @@
 // Two steps. What does not depend on the path - per draft position the K largest raw logits in
 // (value descending, id ascending) order and the row's log-sum-exp - is one pass over all
 // slots' rows: arcs_logprobs_batch. The path itself is sequential over the (at most 7)
-// positions of a slot, because a position's scores depend on the token chosen before it: one
-// warp per slot walks it, a candidate to a lane. A candidate's score is accumulated exactly as
+// positions of a slot, because a position's scores depend on the token chosen before it. But that
+// token is one of the K candidates of the position before: the winners for all of them are worked
+// out first, all positions at once (dflash_score_kernel), and the walk only looks them up
+// (dflash_walk_kernel). Where that would be too much work (many slots, large K and rank) one
+// warp per slot walks and scores, a candidate to a lane (dflash_path_kernel). A candidate's score is accumulated exactly as
 // the reference does (:489-493): float products, added one by one in index order to a double
 // that starts at the logit, so that the comparison of scores falls as it does there.
 #include "common.cuh"
@@ -27,6 +30,7 @@ struct DflDev {
   double min_p;
   const int32_t* top_id;  // [slots * nd][K] from the first step
   const double* lse;      // [slots * nd]
+  int32_t* win;           // [slots * nd][K] winner at a position for each candidate of the one before (-1: no score)
   int32_t* n_out;
   int32_t* out_tokens;
   int32_t out_stride;
@@ -112,6 +116,113 @@ __global__ void __launch_bounds__(32) dflash_path_kernel(const DflDev a) {
   if (lane == 0) a.n_out[s] = n_out;
 }
 
+constexpr int kDflThreads = 256;
+constexpr int kDflMaxSteps = 8;
+// words of a codebook row in shared memory: odd, so that a column's K entries lie in different banks
+__host__ __device__ inline int dfl_row_words(int rank) { return ((rank + 1) / 2) | 1; }
+static size_t dfl_score_smem(int K, int rank) { return (size_t)K * K * 8 + (size_t)K * (rank + 1) * 4 + (size_t)K * dfl_row_words(rank) * 4; }
+
+// One CTA per position and slot: every candidate's score after every candidate of the position
+// before (after the slot's token at the first position), a pair to a thread, and the winner for
+// each. What bounds it is one chain of `rank` fp64 additions, once instead of once a position.
+template <typename T>
+__global__ void __launch_bounds__(kDflThreads) dflash_score_kernel(const DflDev a) {
+  extern __shared__ __align__(16) char dfl_smem[];
+  const int K = a.K, rank = a.rank, tid = threadIdx.x;
+  const int s = blockIdx.x / a.steps, t = blockIdx.x % a.steps;
+  const size_t row = (size_t)s * a.nd + t;
+  double* const score = reinterpret_cast<double*>(dfl_smem);                      // [K][K]
+  float* const ph = reinterpret_cast<float*>(score + K * K);                      // [K][rank + 1]
+  uint32_t* const sv = reinterpret_cast<uint32_t*>(ph + (size_t)K * (rank + 1));  // [K][row_words]
+  const int rw = dfl_row_words(rank);
+  const int32_t* ids = a.top_id + row * K;
+  const float* h = a.hproj + row * rank;
+  const int before = t == 0 ? 1 : K;
+  for (int x = tid; x < before * rank; x += kDflThreads) {
+    const int i = x / rank, r = x - i * rank;
+    const int32_t prev = t == 0 ? __ldg(&a.tok[s]) : __ldg(&ids[i - K]);  // (the row before)
+    ph[i * (rank + 1) + r] = prev >= 0 && prev < a.V ? __fmul_rn(bf16_bits(__ldg(&a.pred[(size_t)prev * rank + r])), __ldg(&h[r])) : 0.0f;  // :487
+  }
+  for (int x = tid; x < K * rank; x += kDflThreads) {
+    const int k = x / rank, r = x - k * rank;
+    const int32_t c = __ldg(&ids[k]);
+    reinterpret_cast<uint16_t*>(sv + (size_t)k * rw)[r] = c >= 0 ? __ldg(&a.succ[(size_t)c * rank + r]) : (uint16_t)0;
+  }
+  __syncthreads();
+  const char* l = static_cast<const char*>(a.logits) + row * (size_t)a.row_stride * sizeof(T);
+  for (int x = tid; x < before * K; x += kDflThreads) {
+    const int i = x / K, k = x - i * K;
+    const int32_t c = __ldg(&ids[k]);
+    double sc = -INFINITY;  // (fewer than K numbers in the row: never chosen)
+    if (c >= 0) {
+      sc = (double)raw_logit<T>(l, c);
+      const float* p = ph + i * (rank + 1);
+      const uint32_t* v = sv + (size_t)k * rw;
+      int r = 0;
+#pragma unroll 4
+      for (; r + 1 < rank; r += 2) {
+        const uint32_t w = v[r >> 1];
+        sc = __dadd_rn(sc, (double)__fmul_rn(p[r], __uint_as_float(w << 16)));
+        sc = __dadd_rn(sc, (double)__fmul_rn(p[r + 1], __uint_as_float(w & 0xFFFF0000u)));
+      }
+      if (r < rank) sc = __dadd_rn(sc, (double)__fmul_rn(p[r], __uint_as_float(v[r >> 1] << 16)));
+    }
+    score[x] = sc;
+  }
+  __syncthreads();
+  for (int i = tid; i < before; i += kDflThreads) {
+    double best = -1e300;
+    int bk = -1;
+    for (int k = 0; k < K; ++k)  // :494, the first among equals
+      if (score[i * K + k] > best) {
+        best = score[i * K + k];
+        bk = k;
+      }
+    a.win[row * K + i] = bk;
+  }
+}
+
+// The walk over the winners: one warp per slot; all it may need is fetched at once.
+template <typename T>
+__global__ void __launch_bounds__(32) dflash_walk_kernel(const DflDev a) {
+  __shared__ int32_t win[kDflMaxSteps * kDflMaxK], id[kDflMaxSteps * kDflMaxK];
+  __shared__ float lg[kDflMaxSteps * kDflMaxK];
+  __shared__ double lse[kDflMaxSteps];
+  const int s = blockIdx.x, lane = threadIdx.x, K = a.K;
+  const size_t row0 = (size_t)s * a.nd;
+  for (int x = lane; x < a.steps * K; x += 32) {
+    const int t = x / K;
+    const int32_t c = __ldg(&a.top_id[row0 * K + x]);
+    id[x] = c;
+    win[x] = (t > 0 || x == 0) ? a.win[row0 * K + x] : -1;
+    lg[x] = c >= 0 ? raw_logit<T>(static_cast<const char*>(a.logits) + (row0 + t) * (size_t)a.row_stride * sizeof(T), c) : 0.0f;
+  }
+  if (lane < a.steps) lse[lane] = __ldg(&a.lse[row0 + lane]);
+  __syncwarp();
+  if (lane != 0) return;
+  const int32_t tok = __ldg(&a.tok[s]);
+  double path_p = 1.0;
+  int n_out = 0, i = 0;
+  if (tok < 0 || tok >= a.V) raise_status(a.status, ARCS_ERR_ARG);  // (a token outside the codebooks: nothing can be scored from it)
+  else
+    for (int t = 0; t < a.steps; ++t) {
+      const int k = max(win[t * K + i], 0);  // (no score above -1e300: the best logit, :489)
+      const int32_t bt = id[t * K + k];
+      if (bt < 0) break;  // (a row without a single number)
+      if (a.min_p > 0.0) {  // :496-503
+        const float mx = lg[t * K];  // (the candidates are sorted: the first holds the largest logit)
+        const double z = exp(lse[t] - (double)mx);
+        path_p *= exp((double)lg[t * K + k] - (double)mx) / z;
+        if (a.path_p) a.path_p[row0 + t] = path_p;
+        if (t > 0 && path_p < a.min_p) break;  // (the first draft always goes)
+      }
+      a.out_tokens[(size_t)s * a.out_stride + n_out] = bt;
+      ++n_out;
+      i = k;
+    }
+  a.n_out[s] = n_out;
+}
+
 static size_t up256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 }  // namespace arcs
@@ -121,7 +232,7 @@ extern "C" size_t arcs_dflash_workspace_bytes(int32_t slots, int32_t nd, int32_t
   if (slots <= 0 || nd <= 0 || V <= 0 || topk <= 0) return 0;
   const int K = topk < V ? topk : V;
   const size_t R = (size_t)slots * nd;
-  return up256(arcs_logprobs_workspace_bytes((int32_t)R, V, K)) + up256(R * K * 4) + up256(R * K * 8) + up256(R * 8);
+  return up256(arcs_logprobs_workspace_bytes((int32_t)R, V, K)) + 2 * up256(R * K * 4) + up256(R * K * 8) + up256(R * 8);
 }
 
 extern "C" int arcs_dflash_select(const arcs_dflash_args* g, void* stream) {
@@ -183,6 +294,24 @@ extern "C" int arcs_dflash_select(const arcs_dflash_args* g, void* stream) {
   a.out_stride = g->out_stride;
   a.path_p = g->path_p;
   a.status = g->status;
+  a.win = reinterpret_cast<int32_t*>(p + lp_bytes + up256(R * K * 4) + up256(R * K * 8) + up256(R * 8));
+  // All pairs scored first while that is little work for the whole GPU: with the walk a call
+  // of 8 slots x 7 positions, K 16, rank 256 goes 78 -> 62 us, a warp per slot scoring as it goes -> this
+  const size_t smem = dfl_score_smem(K, a.rank);
+  if (a.steps >= 1 && a.steps <= kDflMaxSteps && smem <= 160 * 1024 && (double)g->slots * a.steps * K * K * a.rank <= 64e6) {
+#define ARCS_LAUNCH(T)                                                                                        \
+  do {                                                                                                        \
+    static std::atomic<unsigned long long> attr_done{0};                                                      \
+    const cudaError_t e = ensure_dynamic_smem(dflash_score_kernel<T>, 160 * 1024, attr_done);                 \
+    if (e != cudaSuccess) return set_error(ARCS_ERR_CUDA, cudaGetErrorString(e));                             \
+    dflash_score_kernel<T><<<(unsigned)(g->slots * a.steps), kDflThreads, smem, st>>>(a);                     \
+    dflash_walk_kernel<T><<<(unsigned)g->slots, 32, 0, st>>>(a);                                              \
+  } while (0)
+    if (g->dtype == ARCS_F32) ARCS_LAUNCH(float);
+    else ARCS_LAUNCH(__nv_bfloat16);
+#undef ARCS_LAUNCH
+    return check_launch("dflash_select");
+  }
   if (g->dtype == ARCS_F32) dflash_path_kernel<float><<<(unsigned)g->slots, 32, 0, st>>>(a);
   else dflash_path_kernel<__nv_bfloat16><<<(unsigned)g->slots, 32, 0, st>>>(a);
   return check_launch("dflash_select");
