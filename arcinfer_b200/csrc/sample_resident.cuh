@@ -285,6 +285,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   __syncthreads();
   if (s.cnt > kResCap) {
     // too many (masses of equal logits, a handful of elements a thread): the k best, exactly, by pushes and prunes
+    __syncthreads();  // (every thread has read the count that brings it here, before it is set to zero)
     if (tid == 0) {
       s.cnt = 0;
       s.tau = 0ull;

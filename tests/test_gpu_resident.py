@@ -64,6 +64,29 @@ def test_equal_and_infinite_logits(bf16):
     assert 0 <= out["token"][2] < 7
 
 
+@pytest.mark.parametrize("V", [1100, 1536, 2047, 60000])
+def test_slices_that_overflow(V):
+    """more candidates than a slice keeps: narrow rows give fewer chunks than the 256 wanted, so that
+    no threshold is found; equal and infinite logits all reach theirs. Many rows, again and again: the
+    threads of a slice must all go the same way"""
+    from gpuutil import check_rows, run_gpu_sample
+
+    g = np.random.default_rng(V)
+    B = 24
+    x = (g.standard_normal((B, V), dtype=np.float32) * 3).astype(np.float32)
+    x[::3] = 0.5
+    x[1::6] = -np.inf
+    x[1::6, V // 2] = 1.0
+    xb = synth.f32_to_bf16_bits(x)
+    params = synth.make_params(B, top_k=256, top_p=1.0)
+    us = g.random(B)
+    first = run_gpu_sample(xb, True, params, None, us)
+    check_rows(first, xb, True, params, None, us)
+    for _ in range(20):
+        again = run_gpu_sample(xb, True, params, None, us)
+        assert all(np.array_equal(again[k], first[k]) for k in ("token", "n_cand", "cand_id"))
+
+
 @pytest.mark.parametrize("V,B", [(151936, 55), (151936, 56), (32000, 222), (32000, 223), (32000, 445)])
 def test_where_the_route_changes(V, B):
     from gpuutil import check_rows, run_gpu_sample
