@@ -63,8 +63,9 @@ __device__ __forceinline__ unsigned long long cluster_ld64(const void* p, uint32
   asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr(p, rank)) : "memory");
   return v;
 }
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// (not the aligned forms: these stand behind code that a warp's lanes leave at different times)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
 
 template <typename T>
 __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_constant__ SampleDev a, int ctas, int slice) {
