@@ -225,7 +225,13 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
     }
   }
   const float sc = tid < sc_n ? __uint_as_float(s.scal[tid]) : NAN;
-  if (!ok) s.failed = 1;
+  if (!ok) {
+    // a copy did not land in time: all that were issued get one more bounded wait, so that none is
+    // still on its way when the CTA gives its shared memory up
+    for (int i = 0; i < kResParts; ++i)
+      if (i * part < nchunk) mbar_wait_warp(&s.bars[i], 0u);
+    s.failed = 1;
+  }
   const int kB = r.kB;
   const bool few = kB <= 64;  // one maximum a thread gives a tight threshold
   {
