@@ -111,41 +111,60 @@ template <> struct LpElem<__nv_bfloat16> {
 // chunks in fp64. The reference is at least every element the thread has seen: the terms that make
 // up a peaked sum are exact ones. Against fp64 sums the log of a row's sum has an rms error of
 // 0.9e-8 (fp32 normal logits, 512 rows of 151936; 1.1e-8 when exponents were rounded twice).
+// That holds while c's own rounding is small: up to |ref| = 2^24 it is at most 1. Beyond (logits masked
+// with a large negative number, above all) and while there is no reference, c is a NaN: every term
+// is then one too, the tile's sum is made by lp_tile_slow relative to ref itself, and S means that.
+constexpr float kLpNear = 16777216.0f;
+__device__ __forceinline__ float lp_c(float ref) { return fabsf(ref) <= kLpNear ? __fmul_rn(ref, kL2e) : NAN; }
 struct LpSum {
-  float ref = -INFINITY, c = -INFINITY;
+  float ref = -INFINITY, c = NAN;
   double S = 0.0;
-  __device__ __forceinline__ double off() const { return (double)ref * (double)kL2e - (double)c; }  // exact: what the terms' exponents are short of
-  __device__ __forceinline__ double scaled() const { return S == 0.0 ? 0.0 : S * exp2(-off()); }    // sum of exp(l - ref)
+  __device__ __forceinline__ double off() const { return c == c ? (double)ref * (double)kL2e - (double)c : 0.0; }  // exact: what the terms' exponents are short of
+  __device__ __forceinline__ double scaled() const { return S == 0.0 ? 0.0 : S * exp2(-off()); }                   // sum of exp(l - ref)
   // a new, larger reference
   __device__ __forceinline__ void raise(float m) {
-    const float cm = __fmul_rn(m, kL2e);
-    if (S != 0.0) S *= exp2((double)c - (double)cm);
+    const LpSum from = *this;
     ref = m;
-    c = cm;
+    c = lp_c(m);
+    if (S == 0.0) return;
+    if (c == c && from.c == from.c) S *= exp2((double)from.c - (double)c);
+    else S = from.scaled() * exp((double)from.ref - (double)m) * exp2(off());
+  }
+  // exp(v - ref) in fp64, without the exponential where it has no digits or is one
+  __device__ __forceinline__ double term(float v) const {
+    const double d = (double)v - (double)ref;
+    return v != v || d < -750.0 ? 0.0 : d == 0.0 ? 1.0 : exp(d);
   }
   // one more value, in the slow way
   __device__ __forceinline__ void one(float v) {
     if (v > ref) raise(v);
-    if (ref > -INFINITY && v == v) S += exp((double)v - (double)ref) * exp2(off());
+    if (ref > -INFINITY) S += term(v) * exp2(off());
   }
 };
 // The rare steps of the main loop are calls: what they need in registers is then spilled around
 // them and not in the loop itself.
-__device__ __noinline__ double lp_rescale(double S, float c, float cm) { return S * exp2((double)c - (double)cm); }
-// (the thread's chunks first, first + kLpThreads, ... of a piece with nchunk of them at body, read once more)
-template <typename T>
-__device__ __noinline__ double lp_tile_slow(double S, float ref, float c, const char* body, int first, int nchunk) {
+__device__ __noinline__ double lp_rescale(double S, float ref, float m) {
   LpSum s;
   s.S = S;
   s.ref = ref;
-  s.c = c;
+  s.c = lp_c(ref);
+  s.raise(m);
+  return s.S;
+}
+// (the thread's chunks first, first + kLpThreads, ... of a piece with nchunk of them at body, read once more)
+template <typename T>
+__device__ __noinline__ double lp_tile_slow(double S, float ref, const char* body, int first, int nchunk) {
+  LpSum s;
+  s.ref = ref;
+  s.c = lp_c(ref);
+  double z = 0.0;
   const int end = min(nchunk, first + kLpChunks * kLpThreads);
   for (int i = first; i < end; i += kLpThreads) {
     const uint4 q = ldg128_stream(body + (size_t)i * 16);
 #pragma unroll
-    for (int e = 0; e < Elem<T>::kPerChunk; ++e) s.one(Elem<T>::get(q, e));  // (none exceeds the reference)
+    for (int e = 0; e < Elem<T>::kPerChunk; ++e) z += s.term(Elem<T>::get(q, e));  // (none exceeds the reference)
   }
-  return s.S;
+  return S + z * exp2(s.off());
 }
 // What the threads have published of their own maxima belongs to disjoint sets of elements, so the
 // n-th largest of it is a lower bound of the n-th largest element: the threshold (a key,
@@ -512,14 +531,13 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
         for (int w = 1; w < kLpThreads / 32; ++w) mk = max(mk, sh.wkey[w]);
         if (mk != 0u) {
           sum.ref = value_of(mk);
-          sum.c = __fmul_rn(sum.ref, kL2e);
+          sum.c = lp_c(sum.ref);
         }
         if (TOP && tid < 32) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
       } else if (tm > sum.ref) {
-        const float cm = __fmul_rn(tm, kL2e);
-        if (sum.S != 0.0) sum.S = lp_rescale(sum.S, sum.c, cm);
+        if (sum.S != 0.0) sum.S = lp_rescale(sum.S, sum.ref, tm);
         sum.ref = tm;
-        sum.c = cm;
+        sum.c = lp_c(tm);
       }
       // ---- the sum of exponentials
       {
@@ -537,8 +555,8 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
         }
         if ((z[0] + z[1]) + (z[2] + z[3]) < 1e30f) {
           sum.S += (widen_pos(z[0]) + widen_pos(z[1])) + (widen_pos(z[2]) + widen_pos(z[3]));
-        } else {
-          sum.S = lp_tile_slow<T>(sum.S, sum.ref, sum.c, p.body, t * kLpChunks * kLpThreads + tid, nchunk);  // (a NaN, an infinity, or nothing but -inf so far)
+        } else if (sum.ref > -INFINITY) {  // (nothing but -inf so far: nothing to add)
+          sum.S = lp_tile_slow<T>(sum.S, sum.ref, p.body, t * kLpChunks * kLpThreads + tid, nchunk);  // (a NaN, an infinity, or a reference far from zero)
         }
       }
       // ---- a tile that may hold one of the n best is noted, to be looked into at the piece's end
