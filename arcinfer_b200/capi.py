@@ -111,6 +111,8 @@ def _ptr(t):
 
 def _stream(device):
     """the raw handle of torch's current stream of the device (without the stream object around it)"""
+    if device.type != "cuda":
+        raise ValueError(f"Expected a cuda device, but got: {device}")
     i = device.index
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if i is None else i)
 
