@@ -65,6 +65,8 @@ lib.arcs_sample_workspace_bytes.restype = C.c_size_t
 lib.arcs_sample_workspace_bytes.argtypes = [C.c_int32, C.c_int32, C.c_int32, C.c_int32]
 lib.arcs_sample_batch.restype = C.c_int
 lib.arcs_sample_batch.argtypes = [C.POINTER(SampleArgs), C.c_void_p]
+lib.arcs_sample_launches.restype = C.c_int
+lib.arcs_sample_launches.argtypes = [C.c_int32] * 6
 
 
 class MergeArgs(C.Structure):

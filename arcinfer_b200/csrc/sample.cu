@@ -88,6 +88,11 @@ static ResPlan plan_resident(int B, int V, int elt, int max_hist, int max_bias) 
   if (p.ctas && (int64_t)B * p.ctas * 2 > 3 * kSmCount * std::min<int64_t>(per_sm, 2)) p.ctas = 0;
   return p;
 }
+extern "C" int arcs_sample_launches(int32_t B, int32_t V, int32_t dtype, int32_t masked, int32_t max_hist, int32_t max_bias) {
+  if (B <= 0 || V <= 0 || max_hist < 0 || max_bias < 0 || (dtype != ARCS_F32 && dtype != ARCS_BF16)) return 0;
+  return !masked && plan_resident(B, V, dtype == ARCS_F32 ? 4 : 2, max_hist, max_bias).ctas > 0 ? 1 : 2;
+}
+
 template <typename T>
 static cudaError_t launch_resident(const SampleDev& a, const ResPlan& p, cudaStream_t st) {
   static std::atomic<unsigned long long> attr_done{0};

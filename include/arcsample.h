@@ -121,6 +121,9 @@ typedef struct {
 /* max_list: max_hist + max_bias of the call (0 without lists) */
 size_t arcs_sample_workspace_bytes(int32_t B, int32_t V, int32_t masked, int32_t max_list);
 int arcs_sample_batch(const arcs_sample_args* args, void* stream);
+/* Kernels such a call launches: 1 where its rows are held on the chip, 2 otherwise (0: bad sizes).
+ * max_hist, max_bias: those of the call, 0 for a list that is not given. */
+int arcs_sample_launches(int32_t B, int32_t V, int32_t dtype, int32_t masked, int32_t max_hist, int32_t max_bias);
 /* Measurement aid: the same launches, one after the other (the finish kernel does not run
  * beside the stream kernel here), with CUDA events between them on `stream`; waits for them and
  * returns the device time of the stream and finish kernels in ms2[0..1] (of the one kernel, and

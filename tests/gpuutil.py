@@ -27,7 +27,8 @@ def widen(x, bf16):
     return synth.bf16_bits_to_f32(x) if bf16 else x
 
 
-def run_gpu_sample(x, bf16, params, hists, us, biases=None, masks=None, mask_row=None, stride=None, offset=0, want_cands=True):
+def run_gpu_sample(x, bf16, params, hists, us, biases=None, masks=None, mask_row=None, stride=None, offset=0, want_cands=True, max_hist=0):
+    """max_hist: a bound above the longest history given (it takes part in the choice of the route)"""
     B = x.shape[0]
     lg, V = to_dev_logits(x, bf16, stride, offset)
     p = ab.capi.params_to_device(params, "cuda")
@@ -36,7 +37,7 @@ def run_gpu_sample(x, bf16, params, hists, us, biases=None, masks=None, mask_row
     if hists is not None:
         ho, hi = synth.csr(hists)
         kw.update(hist_off=torch.from_numpy(ho).cuda(), hist_ids=torch.from_numpy(hi).cuda() if len(hi) else torch.zeros(1, dtype=torch.int32, device="cuda"),
-                  max_hist=int(max(len(h) for h in hists)))
+                  max_hist=max(max_hist, int(max(len(h) for h in hists))))
     if biases is not None:
         bo, bi = synth.csr([[b[0] for b in bl] for bl in biases])
         bv = np.array([b[1] for bl in biases for b in bl], np.float32)

@@ -1,7 +1,7 @@
 """Rows held whole on the chip: sizes about a slice's and a cluster's borders, unaligned rows, lists
 that repeat ids, k from 1 to 256, rows that overflow a slice's candidates (masses of equal
-logits), vocabulary shards, and the number of rows at which the call changes to the streaming
-kernels. Ids, counts and adjusted logits bit-exact against the CPU oracle, probabilities within
+logits), and the number of rows at which the call changes to the streaming kernels (the columns of
+vocabulary shards: test_gpu_vocab_shard.py). Ids, counts and adjusted logits bit-exact against the CPU oracle, probabilities within
 1e-6 (the last rounding of a float exponential: 2^-24, with the same sums in the same order)."""
 import numpy as np
 import pytest
