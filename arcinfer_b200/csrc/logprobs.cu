@@ -1,21 +1,21 @@
 // logprobs_batch: per row the log-softmax of one token and the top_n largest raw logits as log
 // probabilities (tools/server_chat.h:417-441; zero/runz.cpp:478-484 scores perplexity with the
-// same sum). One launch, one pass. The rows, cut into units of columns, are dealt out to the CTAs in
-// equal runs of consecutive units (lp_plan): a CTA takes the end of one row, some whole rows and
-// the beginning of another, so that no wave of CTAs is left half empty and a row is cut only where
-// one CTA's share ends. Every such piece of a row is read once, straight into registers (a tile of
+// same sum). One launch, one pass. Many rows: a CTA to a row. Fewer: the rows, cut into units of
+// columns, are dealt out to the CTAs in equal runs of consecutive units (lp_plan): a CTA takes the end
+// of one row, some whole rows and the beginning of another, so that a row is cut only where one CTA's
+// share ends. Every such piece of a row is read once, straight into registers (a tile of
 // four 16-byte chunks a thread, the next tile's loads in flight while one is worked on), and gives
 //  - per thread a sum of exponentials relative to a reference value of the thread's own, in fp64;
 //  - notes of the threads' tiles that may hold one of the top_n largest elements, which are read
 //    again at the piece's end.
-// After a piece's first tile no thread waits for another. The CTA that finishes a row last merges its pieces
-// (left in the workspace) and writes the row's output.
+// After a piece's first tile no thread waits for another. The CTA that finishes a cut row last merges its
+// pieces (left in the workspace) and writes the row's output.
 //
 // What bounds it: memory, then the special-function unit (one ex2 per logit, 16 a clock and SM:
-// 59 us for 1024 x 262144, next to 82 us for its 537 MB); what the kernel takes on top are the pieces'
-// ends and beginnings. 1024 x 262144 bf16: 20 alternatives 226 -> 151 us, none 140 -> 104 us; 512 x 151936
-// fp32, none: 84 -> 57 us (a CTA per row through a shared-memory ring with two barriers a tile, the
-// candidates' buffer kept by the whole CTA, -> this).
+// 59 us for 1024 x 262144, next to 83 us for its 537 MB); what the kernel takes on top are the pieces'
+// ends and beginnings. 1024 x 262144 bf16: 20 alternatives 216 -> 140 us, none 134 -> 113 us; 512 x
+// 151936 fp32, none: 80 -> 59 us (a row through a shared-memory ring with two barriers a tile, the
+// candidates' buffer kept by the whole CTA, -> this; graph replays).
 #include <algorithm>
 
 #include "plan.h"
@@ -603,19 +603,31 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
 
 using namespace arcs;
 
-// How B rows of V columns are dealt out: units of `unit` columns (a multiple of 2048, at most
-// kMaxSeg to a row), in equal runs to the CTAs, which all fit the GPU at once. 1024 rows as one CTA
-// each are 1.4 waves of 740; dealt out evenly they are one. A row's units lie with at most
-// max_pieces CTAs.
+// Rows enough for the GPU, or short ones, are not cut: a row to a CTA, nothing handed over and no
+// workspace used, so that such calls may overlap as they like. (Cutting them too, and dealing the
+// pieces out evenly, was measured: none wanted, 512 x 151936 fp32 53 us against 59, 1024 x 262144
+// bf16 99 against 113; 20 alternatives 75 / 74 and 139 / 140, 600 x 50000 bf16 39 / 27.)
+constexpr int32_t kLpManyRows = 3 * kSmCount, kLpShortRow = 8192;
+static bool lp_whole(int32_t B, int32_t V) { return B >= kLpManyRows || V <= kLpShortRow; }
+// How B rows of V columns are dealt out: whole, or cut into units of `unit` columns (a multiple of
+// 2048, at most kMaxSeg to a row) that are given in equal runs to the CTAs, which all fit the GPU at
+// once: a row is cut only where one CTA's share ends. A row's units lie with at most max_pieces CTAs.
 struct LpPlan {
   int32_t unit, row_units, max_pieces;
   uint32_t run, longer;
   unsigned grid;
 };
-static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n, bool whole) {
+static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n) {
   LpPlan p;
+  if (lp_whole(B, V)) {
+    p.unit = V;
+    p.row_units = p.max_pieces = 1;
+    p.run = 1;
+    p.longer = 0;
+    p.grid = (unsigned)B;
+    return p;
+  }
   p.unit = std::max(2048, ((V - 1) / kMaxSeg + 2048) / 2048 * 2048);
-  if (whole || (int64_t)B * kMaxSeg > INT32_MAX) p.unit = V;
   p.row_units = (V + p.unit - 1) / p.unit;
   const uint32_t total = (uint32_t)B * (uint32_t)p.row_units;
   p.grid = std::min<uint32_t>(total, kSmCount * lp_per_sm(top_n > 0));
@@ -627,7 +639,8 @@ static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n, bool whole) {
 
 extern "C" size_t arcs_logprobs_workspace_bytes(int32_t B, int32_t V, int32_t top_n) {
   if (B <= 0 || V <= 0 || top_n < 0) return 0;
-  const LpPlan p = lp_plan(B, V, top_n, false);
+  if (lp_whole(B, V)) return 16;  // (not used)
+  const LpPlan p = lp_plan(B, V, top_n);
   return 256 + (((size_t)B * 4 + 255) & ~(size_t)255) + (size_t)B * p.max_pieces * (sizeof(LpPart) + (size_t)top_n * 8);
 }
 
@@ -644,11 +657,7 @@ extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
   a.row_stride = g->row_stride;
   a.B = g->B;
   a.V = g->V;
-  // (444 rows or more, or short rows: served without a workspace too, a row to a unit)
-  int nseg, seg_len;
-  plan_segments(g->B, g->V, &nseg, &seg_len, 3);
-  const bool no_ws = nseg == 1 && (!g->workspace || g->workspace_bytes < arcs_logprobs_workspace_bytes(g->B, g->V, g->top_n));
-  const LpPlan plan = lp_plan(g->B, g->V, g->top_n, no_ws);
+  const LpPlan plan = lp_plan(g->B, g->V, g->top_n);
   a.unit = plan.unit;
   a.row_units = plan.row_units;
   a.run = plan.run;
@@ -665,7 +674,7 @@ extern "C" int arcs_logprobs_batch(const arcs_logprob_args* g, void* stream) {
   a.ws_ctr = nullptr;
   a.ws_part = nullptr;
   a.ws_list = nullptr;
-  if (!no_ws) {
+  if (!lp_whole(g->B, g->V)) {
     if (!g->workspace || g->workspace_bytes < arcs_logprobs_workspace_bytes(g->B, g->V, g->top_n))
       return set_error(ARCS_ERR_WORKSPACE, "logprobs_batch: workspace too small");
     if ((reinterpret_cast<uintptr_t>(g->workspace) & 15u) != 0) return set_error(ARCS_ERR_WORKSPACE, "logprobs_batch: workspace must be 16-byte aligned");

@@ -311,8 +311,10 @@ void arcs_jcon_destroy(arcs_jcon* h);
  * logprobs_batch: per row, the log probability of one token and the top_n most likely
  * alternatives, from the RAW logits (no penalty, no bias): the `logprobs` entry of
  * tools/server_chat.h:417-441, and the log-softmax that scores perplexity and KL
- * (zero/runz.cpp:478-484, :639-646). One pass over the logits, one launch. The rows are dealt out
- * evenly to the SMs; where a row is cut, its pieces' results meet in the workspace.
+ * (zero/runz.cpp:478-484, :639-646). One pass over the logits, one launch. When there are few
+ * rows they are cut, and a row's pieces meet in the workspace: such calls need one, and calls that
+ * may overlap (on two streams, in a captured graph and beside it) need one each. Calls of 444 rows
+ * or more, or of at most 8192 columns, use none.
  *   mx = max; z = sum exp(l - mx) accumulated in fp64; lse = mx + log(z);
  *   logprob[b] = l[token[b]] - lse;  top_id / top_logprob: the top_n largest logits, best first
  *   (equal logits: lower id first), as log probabilities.
@@ -333,7 +335,7 @@ typedef struct {
   double* lse;            /* [B] optional: log of the sum of exponentials */
   int32_t* top_id;        /* [B][top_stride]; entries past min(top_n, V) are not written */
   double* top_logprob;    /* [B][top_stride] */
-  void* workspace;        /* arcs_logprobs_workspace_bytes(), zeroed before its first use and again before a call of another shape (B, V, top_n) takes it over */
+  void* workspace;        /* arcs_logprobs_workspace_bytes(), 16-byte aligned, zeroed before its first use and again before a call of another shape (B, V, top_n) takes it over; may be NULL where rows are not cut */
   size_t workspace_bytes;
   int32_t* status;        /* device status word (first error wins), may be NULL */
 } arcs_logprob_args;

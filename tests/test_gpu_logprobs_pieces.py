@@ -1,8 +1,11 @@
 """arcs_logprobs_batch where its rows are cut and its thresholds are odd: rows whose pieces end on
 and beside a unit's border, one and several rows to a CTA, rows of mostly -inf or NaN, many
 alternatives; and the call without a workspace. Against the CPU oracle: ids bit-exact, log
-probabilities within 1e-6 (a term's error is below 2^-21: two roundings of 2^-24 of an exponent
-below 8, and 2^-22.5 of the special-function unit; a sum's is no larger)."""
+probabilities within 1e-6. A term's exponent x = (l - ref) * log2 e is rounded once, to 2^-24 |x|, which
+is 2^-24.5 |x| of the term; the special-function unit adds 2^-22.5, the fp32 sums over a chunk 3 * 2^-24.
+Weighted by the terms' shares of the sum the |x| come to 12.5 at most with 131073 of them (one term of a
+tenth of the sum, all others alike), so that the sum, and with it its logarithm, is within 8.7e-7 even
+if no two errors cancel."""
 import ctypes as C
 
 import numpy as np
@@ -89,3 +92,26 @@ def test_without_workspace():
         assert torch.equal(got["top_id"], want["top_id"]) and torch.allclose(got["lse"], want["lse"], rtol=0, atol=TOL)
     a.B, a.V, a.row_stride = 3, 8193, 8193
     assert ab.lib.arcs_logprobs_batch(C.byref(a), None) != 0
+
+
+@pytest.mark.parametrize("off", [0, 4])
+def test_rows_that_are_not_cut_leave_the_workspace_alone(off):
+    """whatever it holds and wherever it begins: such calls may share one, and overlap"""
+    import arcinfer_b200 as ab
+
+    g = torch.Generator(device="cuda").manual_seed(5)
+    for B, V in ((444, 20000), (1500, 9000), (3, 8192)):
+        lg = torch.from_numpy(_rows(np.random.default_rng(B), B, V, "normal")).cuda()
+        want = ab.logprobs_batch(lg, None, 4)
+        ws = torch.randint(0, 256, (1 << 24,), dtype=torch.uint8, device="cuda", generator=g)
+        kept = ws.clone()
+        got = {"lse": torch.zeros(B, dtype=torch.float64, device="cuda"), "top_id": torch.zeros(B, 4, dtype=torch.int32, device="cuda"),
+               "top_logprob": torch.zeros(B, 4, dtype=torch.float64, device="cuda")}
+        a = ab.capi.LogprobArgs()
+        a.logits, a.dtype, a.B, a.V, a.row_stride, a.top_n, a.top_stride = lg.data_ptr(), 0, B, V, V, 4, 4
+        a.lse, a.top_id, a.top_logprob = (got[k].data_ptr() for k in ("lse", "top_id", "top_logprob"))
+        a.workspace, a.workspace_bytes = ws.data_ptr() + off, ws.numel() - off
+        assert ab.lib.arcs_logprobs_batch(C.byref(a), torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        assert torch.equal(got["top_id"], want["top_id"]) and torch.equal(got["lse"], want["lse"]) and torch.equal(ws, kept)
+        assert ab.lib.arcs_logprobs_workspace_bytes(B, V, 256) == 16
