@@ -35,8 +35,10 @@ constexpr int kLpTileBytes = kLpChunks * kLpThreads * 16;
 constexpr int kLpAhead = 3;                   // tiles ahead of the one worked on that are asked into the L2 cache
 constexpr int kLpFew = 64;                    // up to so many alternatives one maximum per thread gives a tight threshold
 // records a CTA keeps of threads and tiles whose maximum reached the threshold of the moment: one a thread of
-// the first tile, then about as many as alternatives wanted (plus a seventh) each time the piece doubles
+// the first tile, then about as many as alternatives wanted (plus a seventh) each time the piece doubles.
+// Each time another kLpMark have come the threshold is raised out of turn (a masked region has ended).
 template <int TOP> constexpr int kLpRec = TOP == 0 ? 1 : TOP == 1 ? 1024 : 3072;
+template <int TOP> constexpr uint32_t kLpMark = TOP == 0 ? 0 : (kLpRec<TOP> - kLpThreads) / 4;
 
 struct LpPart {      // what a piece leaves for the merge
   double z;          // sum of exp(l - M) over the piece
@@ -175,8 +177,57 @@ __device__ __noinline__ void lp_raise_threshold(const uint32_t* keys, int n, uin
   if ((threadIdx.x & 31) == 0) asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(smem_addr(tkey)), "r"(k) : "memory");
 }
 
-// The n best of a piece read once more, element by element (slow, and rare: the chunks set aside
-// overflowed, with ascending data or masses of equal logits). Called by all threads.
+// The same after the first tile, whose threads are all there: an element of a later tile has a higher
+// id than the n elements found, so that it must exceed the n-th of them, not only reach it. What lies
+// in a region of equal logits (masked ones, -inf among them) is then not noted again tile by tile.
+template <int PER>
+__device__ __noinline__ void lp_first_threshold(const uint32_t* keys, int n, uint32_t* tkey) {
+  const uint32_t k = warp_kth16<PER>(keys, n);
+  uint32_t m = 0xFFFFFFFFu;  // the smallest key at or above that bound: n keys are not below it
+#pragma unroll
+  for (int i = 0; i < PER; ++i) {
+    const uint32_t x = keys[i * 32 + (threadIdx.x & 31)];
+    if (x >= k) m = min(m, x);
+  }
+  m = __reduce_min_sync(0xFFFFFFFFu, m);
+  if ((threadIdx.x & 31) == 0 && k != 0u) asm volatile("red.shared.max.u32 [%0], %1;" ::"r"(smem_addr(tkey)), "r"(m + 1u) : "memory");  // (no bound: fewer than n numbers)
+}
+
+// The n best of the tiles noted, when more of their elements reach the threshold than the buffer
+// holds (masses of equal logits in the first tile). Called by all threads.
+template <typename T>
+__device__ __noinline__ void lp_take_noted(const SegPlan& p, const T* row, const Sel& sel, const PruneScratch& ps, const uint32_t* rec_at, int noted) {
+  constexpr int E = Elem<T>::kPerChunk;
+  const int tid = threadIdx.x, nchunk = p.body_bytes / 16;
+  __syncthreads();
+  if (tid == 0) {
+    *sel.cnt = 0;
+    *sel.tau = 0ull;
+  }
+  __syncthreads();
+  for (int i0 = 0; i0 < noted * kLpChunks; i0 += kLpThreads) {  // (a chunk to a thread)
+    const int i = i0 + tid;
+    const uint32_t r = i < noted * kLpChunks ? rec_at[i / kLpChunks] : 0u;
+    const int ci = i < noted * kLpChunks ? ((int)(r >> 8) * kLpChunks + i % kLpChunks) * kLpThreads + (int)(r & 255u) : nchunk;
+    const uint4 q = ci < nchunk ? ldg128_stream(p.body + (size_t)(uint32_t)ci * 16) : make_uint4(0, 0, 0, 0);
+    const uint32_t tkey = (uint32_t)(*sel.tau >> 32);
+    uint32_t bits = 0;
+#pragma unroll
+    for (int e = 0; e < E; ++e) bits |= (ci < nchunk && key_of(Elem<T>::get(q, e)) >= tkey ? 1u : 0u) << e;
+    push_all<kLpThreads>(sel, ps, bits, [&](int e, uint32_t& ky, int32_t& id) {
+      id = p.body_first + ci * E + e;
+      ky = key_of(Elem<T>::get(q, e));
+    });
+  }
+  const bool hv = tid < p.head_n, tv = tid < p.tail_n;
+  push_all<kLpThreads>(sel, ps, (hv ? 1u : 0u) | (tv ? 2u : 0u), [&](int idx, uint32_t& ky, int32_t& id) {
+    id = idx == 0 ? p.lo + tid : p.tail_first + tid;
+    ky = key_of(Elem<T>::load(row + id));
+  });
+}
+
+// The n best of a piece read once more, element by element (slow, and rare: the notes overflowed,
+// with ascending data). Called by all threads.
 template <typename T>
 __device__ __noinline__ void lp_reread(const SegPlan& p, const T* row, const Sel& sel, const PruneScratch& ps) {
   constexpr int E = Elem<T>::kPerChunk;
@@ -238,7 +289,8 @@ struct LpShared {
   int32_t ti[TOP ? kTmpCap : 1];
   float red_m[kLpThreads / 32];
   uint32_t wkey[kLpThreads / 32];
-  uint32_t tkey;                                        // the threshold (a key, inclusive)
+  uint32_t nkey;                                        // the threshold of the main loop: keys from which on a tile is noted
+  uint32_t tkey;                                        // the piece's last one: keys from which on an element is a candidate
   int rec, cnt, misc[8], flag, cnts[kMaxSeg];
 };
 
@@ -291,9 +343,10 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
     sh.red_m[tid >> 5] = M;
     sh.red_s[tid >> 5] = z;
   }
-  if (TOP) {
+  if (tid == 0) {
+    sh.cnt = sh.misc[0] = 0;
+    sh.tkey = 0u;
   }
-  if (tid == 0) sh.cnt = sh.misc[0] = 0;
   __syncthreads();
   if (TOP && tid < 32) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
   if (TOP) __syncthreads();
@@ -303,6 +356,7 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
     const uint32_t tkey = sh.tkey;
     const float tf = floor_value(tkey);
     const int have = tiles > 0 ? sh.rec : 0;
+    int noted = 0;
     if (have <= kLpRec<TOP>) {
       // the records that reach it, closed up (in place: a round's are all read before any is
       // written, at or before the round's first place)
@@ -323,7 +377,8 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
           sh.bid[at] = id;
         }
       };
-      for (int i = tid; i < sh.misc[0] * kLpChunks; i += kLpThreads) {  // (a chunk to a thread, from the L2 cache as a rule)
+      noted = sh.misc[0];
+      for (int i = tid; i < noted * kLpChunks; i += kLpThreads) {  // (a chunk to a thread, from the L2 cache as a rule)
         const uint32_t r = sh.rec_at[i / kLpChunks];
         const int ci = ((int)(r >> 8) * kLpChunks + i % kLpChunks) * kLpThreads + (int)(r & 255u);
         if (ci >= nchunk) continue;
@@ -336,7 +391,8 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
       if (tv) keep(vt, p.tail_first + tid);
     }
     __syncthreads();
-    if (have > kLpRec<TOP> || sh.cnt > kLpCap) lp_reread<T>(p, row, sel, ps);
+    if (have > kLpRec<TOP>) lp_reread<T>(p, row, sel, ps);
+    else if (sh.cnt > kLpCap) lp_take_noted<T>(p, row, sel, ps, sh.rec_at, noted);
     if (sh.cnt > 512) {
       __syncthreads();
       sel_prune<1, kLpThreads>(sel, n, ps, tid);
@@ -499,11 +555,12 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
     };
     if (tid == 0) {
       sh.rec = kLpThreads;  // (the first tile's records have places of their own)
-      sh.tkey = 0u;
+      sh.nkey = 0u;
     }
 
     const int tiles = (nchunk + kLpChunks * kLpThreads - 1) / (kLpChunks * kLpThreads);
     int point = 1;  // the next tile after which the threads publish their maxima: 1, 3, 7, 15, ...
+    uint32_t mark = kLpThreads + kLpMark<TOP>;  // the number of notes at which the warp does so out of turn
     auto tile = [&](int t, const uint4 (&q)[kLpChunks], uint4 (&nq)[kLpChunks]) {
       if (t + 1 < tiles) fetch(nq, t + 1);
       if (tid == 0 && t + kLpAhead < tiles) prefetch_l2(p.body + (size_t)(t + kLpAhead) * kLpTileBytes, min(kLpTileBytes, p.body_bytes - (t + kLpAhead) * kLpTileBytes));
@@ -521,7 +578,13 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
         const uint32_t wk = __reduce_max_sync(0xFFFFFFFFu, tm > -INFINITY ? key_of(tm) : 0u);
         if ((tid & 31) == 0) sh.wkey[tid >> 5] = wk;
         if (TOP) {
-          publish();
+          // (numbers only, -inf among them where every chunk is one of the row's)
+          const bool whole = nchunk >= kLpChunks * kLpThreads;
+#pragma unroll
+          for (int i = 0; i < OWN; ++i) {
+            const float m = OWN == 1 ? tm : Elem<T>::chunk_max(q[i]);
+            sh.keys[i * kLpThreads + tid] = m > -INFINITY || (whole && m == m) ? key_of(m) : 0u;
+          }
           sh.rec_max[tid] = tm;
           sh.rec_at[tid] = tid;
         }
@@ -533,7 +596,7 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
           sum.ref = value_of(mk);
           sum.c = lp_c(sum.ref);
         }
-        if (TOP && tid < 32) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
+        if (TOP && tid < 32) lp_first_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
       } else if (tm > sum.ref) {
         if (sum.S != 0.0) sum.S = lp_rescale(sum.S, sum.ref, tm);
         sum.ref = tm;
@@ -561,21 +624,24 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
       }
       // ---- a tile that may hold one of the n best is noted, to be looked into at the piece's end
       if (TOP && t > 0) {
-        const uint32_t tk0 = sm_ld_volatile(&sh.tkey);
-        if (tm >= floor_value(tk0)) {
-          const uint32_t at = sm_atomic_add(&sh.rec, 1u);
+        const uint32_t nk = sm_ld_volatile(&sh.nkey);
+        uint32_t at = 0u;
+        if (tm >= floor_value(nk)) {
+          at = sm_atomic_add(&sh.rec, 1u);
           if (at < (uint32_t)kLpRec<TOP>) {
             sh.rec_max[at] = tm;
             sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
           }
         }
-        if (t == point) {
+        const bool many = __any_sync(0xFFFFFFFFu, at >= mark && at < (uint32_t)kLpRec<TOP>);
+        if (t == point || many) {
           // (no barrier: what another warp has not published yet only leaves the threshold lower.
-          //  The warps take turns at raising it.)
+          //  The warps take turns at raising it, but for one that finds many notes.)
           publish();
           __syncwarp();
-          if ((tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.tkey);
-          point = 2 * point + 1;
+          if (many || (tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
+          if (many) mark = __reduce_max_sync(0xFFFFFFFFu, at) + kLpMark<TOP>;
+          if (t == point) point = 2 * point + 1;
         }
       }
     };
