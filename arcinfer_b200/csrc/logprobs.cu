@@ -438,34 +438,43 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
       pc = __ldcg(&src->cnt);
     }
     if (TOP) {
-      // A piece that sent n entries has n at or above its last: nothing below the largest such
-      // entry is among the n best of the row.
-      
+      // The lists are sorted. The n-th largest of their first entries (as many of each as there is
+      // room for) bounds the row's n-th from below; what exceeds it goes through the buffer, all
+      // lists' first entries, then all second ones, until no list has one left.
       if (tid == 0) {
         sh.cnt = 0;
         sh.tau = 0ull;
       }
       if (tid < pieces) sh.cnts[tid] = pc;
       __syncthreads();
-      if (tid < pieces && pc == n)
-        sm_red_max_u64(&sh.tau, __ldcg(&a.ws_list[((size_t)b * a.max_pieces + tid) * n + n - 1]) - 1ull);
+      const unsigned long long* lists = a.ws_list + (size_t)b * a.max_pieces * n;
+#pragma unroll
+      for (int j = 0; j < OWN; ++j) {
+        const int e = j * kLpThreads + tid, x = e / pieces, g = e - x * pieces;
+        sh.keys[e] = x < sh.cnts[g] ? comp_key(__ldcg(&lists[(size_t)g * n + x])) : 0u;
+      }
       __syncthreads();
-      // the pieces' lists go through the buffer, kLpThreads entries at a time
+      if (tid < 32) {
+        const uint32_t k = warp_kth16<OWN * kLpThreads / 32>(sh.keys, n);
+        if (tid == 0 && k != 0u) sh.tau = ((unsigned long long)k << 32) - 1ull;
+      }
+      __syncthreads();
       for (int e0 = 0; e0 < pieces * n; e0 += kLpThreads) {
-        const int e = e0 + tid, g = e / max(n, 1), i = e - g * n;
-        const bool have = e < pieces * n && i < sh.cnts[g];
-        const unsigned long long cm = have ? __ldcg(&a.ws_list[((size_t)b * a.max_pieces + g) * n + i]) : 0ull;
+        const int e = e0 + tid, x = e / pieces, g = e - x * pieces;
+        const unsigned long long cm = x < sh.cnts[g] ? __ldcg(&lists[(size_t)g * n + x]) : 0ull;
+        const bool have = cm > sh.tau;
+        if (!__syncthreads_or(have)) break;  // (kLpThreads entries hold one of every list at least)
         push_all<kLpThreads>(sel, ps, have ? 1u : 0u, [&](int, uint32_t& ky, int32_t& id) {
           ky = comp_key(cm);
           id = comp_id(cm);
         });
       }
       __syncthreads();
-      if (sh.cnt > 512) sel_prune<1, kLpThreads>(sel, n, ps, tid);
+      if (sh.cnt > 256) sel_prune<1, kLpThreads>(sel, n, ps, tid);
       __syncthreads();
       c = min(sh.cnt, kLpCap);
     }
-    static_assert(kMaxSeg <= 64, "the pieces' sums lie with two warps");
+    static_assert(kMaxSeg <= 64 && kMaxSeg <= kLpThreads, "the pieces' sums lie with two warps");
     if (tid < 64) {
       warp_lse(pm, pz);
       if ((tid & 31) == 0) {
@@ -678,6 +687,10 @@ static bool lp_whole(int32_t B, int32_t V) { return B >= kLpManyRows || V <= kLp
 // How B rows of V columns are dealt out: whole, or cut into units of `unit` columns (a multiple of
 // 2048, at most kMaxSeg to a row) that are given in equal runs to the CTAs, which all fit the GPU at
 // once: a row is cut only where one CTA's share ends. A row's units lie with at most max_pieces CTAs.
+// Where that would be less than kLpOwnPiece columns a CTA, no CTA gets the end of one row and the
+// beginning of the next, which would cost it a second piece's fixed time (7 us with alternatives: 56 x
+// 30000 fp32, 5 alternatives, 20 us when runs straddle rows, 15 before): a unit to a CTA.
+constexpr int32_t kLpOwnPiece = 8192;
 struct LpPlan {
   int32_t unit, row_units, max_pieces;
   uint32_t run, longer;
@@ -693,10 +706,12 @@ static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n) {
     p.grid = (unsigned)B;
     return p;
   }
-  p.unit = std::max(2048, ((V - 1) / kMaxSeg + 2048) / 2048 * 2048);
+  const int32_t ctas = kSmCount * lp_per_sm(top_n > 0);
+  const int32_t most = (int64_t)B * V < (int64_t)ctas * kLpOwnPiece ? std::min(kMaxSeg, std::max(1, ctas / B)) : kMaxSeg;
+  p.unit = std::max(2048, ((V - 1) / most + 2048) / 2048 * 2048);
   p.row_units = (V + p.unit - 1) / p.unit;
   const uint32_t total = (uint32_t)B * (uint32_t)p.row_units;
-  p.grid = std::min<uint32_t>(total, kSmCount * lp_per_sm(top_n > 0));
+  p.grid = std::min<uint32_t>(total, (uint32_t)ctas);
   p.run = total / p.grid;
   p.longer = total % p.grid;
   p.max_pieces = (int32_t)std::min<uint32_t>(p.row_units, ((uint32_t)p.row_units - 1 + p.run - 1) / p.run + 1);

@@ -29,7 +29,8 @@ def test_regions_of_equal_logits(bf16, top_n, B, V):
         x[7, : V // 3] = np.linspace(1, 2, V // 3)                                     # rising, then level
         if bf16:
             x = synth.bf16_bits_to_f32(synth.f32_to_bf16_bits(x))
-        _check(x, bf16, top_n, range(8))
+        # (row 4 is -inf throughout when one is wanted at that level: its sum is not defined, log 0 - inf)
+        _check(x, bf16, top_n, [r for r in range(8) if not (r == 4 and top_n == 1 and level == -np.inf)])
         if B > 400:
             _check(x[::-1].copy(), bf16, top_n, range(B - 8, B))
 
