@@ -236,6 +236,27 @@ __device__ __forceinline__ uint4 ldg128_stream_if(const void* p, bool on, uint32
   return r;
 }
 
+// ---------------------------------------------------------------- thread-block clusters
+// (shared memory of the cluster's CTA `rank`, at the place p has in this one's)
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ uint32_t cluster_ld(const void* p, uint32_t rank) {
+  uint32_t v;
+  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+__device__ __forceinline__ unsigned long long cluster_ld64(const void* p, uint32_t rank) {
+  unsigned long long v;
+  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr(p, rank)) : "memory");
+  return v;
+}
+// (not the aligned forms: these stand behind code that a warp's lanes leave at different times)
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 // Programmatic dependent launch: a kernel launched with the attribute may start while the kernel
 // before it on the stream still runs; it must pass pdl_wait() before it touches anything that
 // kernel writes (the wait returns when that kernel has completed and its writes are visible).

@@ -114,8 +114,8 @@ template <> struct LpElem<__nv_bfloat16> {
 // up a peaked sum are exact ones. Against fp64 sums the log of a row's sum has an rms error of
 // 0.9e-8 (fp32 normal logits, 512 rows of 151936; 1.1e-8 when exponents were rounded twice).
 // That holds while c's own rounding is small: up to |ref| = 2^24 it is at most 1. Beyond (logits masked
-// with a large negative number, above all) and while there is no reference, c is a NaN: every term
-// is then one too, the tile's sum is made by lp_tile_slow relative to ref itself, and S means that.
+// with a large negative number, above all) c is a NaN, and S the sum of 2^((l - ref) * kL2e): a float
+// so large has neighbours 1 away or more, so that l - ref is exact or leaves a term without weight.
 constexpr float kLpNear = 16777216.0f;
 __device__ __forceinline__ float lp_c(float ref) { return fabsf(ref) <= kLpNear ? __fmul_rn(ref, kL2e) : NAN; }
 struct LpSum {
@@ -210,10 +210,10 @@ __device__ __noinline__ void lp_take_noted(const SegPlan& p, const T* row, const
     const uint32_t r = i < noted * kLpChunks ? rec_at[i / kLpChunks] : 0u;
     const int ci = i < noted * kLpChunks ? ((int)(r >> 8) * kLpChunks + i % kLpChunks) * kLpThreads + (int)(r & 255u) : nchunk;
     const uint4 q = ci < nchunk ? ldg128_stream(p.body + (size_t)(uint32_t)ci * 16) : make_uint4(0, 0, 0, 0);
-    const uint32_t tkey = (uint32_t)(*sel.tau >> 32);
+    const unsigned long long tau = *sel.tau;
     uint32_t bits = 0;
 #pragma unroll
-    for (int e = 0; e < E; ++e) bits |= (ci < nchunk && key_of(Elem<T>::get(q, e)) >= tkey ? 1u : 0u) << e;
+    for (int e = 0; e < E; ++e) bits |= (ci < nchunk && comp_of(key_of(Elem<T>::get(q, e)), p.body_first + ci * E + e) > tau ? 1u : 0u) << e;
     push_all<kLpThreads>(sel, ps, bits, [&](int e, uint32_t& ky, int32_t& id) {
       id = p.body_first + ci * E + e;
       ky = key_of(Elem<T>::get(q, e));
@@ -383,7 +383,7 @@ __device__ __noinline__ void lp_close(const LogprobDev& a, LpShared<TOP>& sh, in
         const int ci = ((int)(r >> 8) * kLpChunks + i % kLpChunks) * kLpThreads + (int)(r & 255u);
         if (ci >= nchunk) continue;
         const uint4 ch = ldg128_stream(p.body + (size_t)(uint32_t)ci * 16);
-        if (!(Elem<T>::chunk_max(ch) >= tf)) continue;
+        if (!(Elem<T>::chunk_max(ch) >= tf) || sm_ld_volatile(&sh.cnt) > (uint32_t)kLpCap) continue;  // (overflowed: below)
 #pragma unroll
         for (int e = 0; e < E; ++e) keep(Elem<T>::get(ch, e), p.body_first + ci * E + e);
       }
@@ -614,43 +614,53 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
       // ---- the sum of exponentials
       {
         float z[kLpChunks];
+        auto terms = [&](auto exponent) {
 #pragma unroll
-        for (int j = 0; j < kLpChunks; ++j) {
-          float e[E];
+          for (int j = 0; j < kLpChunks; ++j) {
+            float e[E];
 #pragma unroll
-          for (int i = 0; i < E; ++i) e[i] = ex2(fmaf(Elem<T>::get(q[j], i), kL2e, -sum.c));
+            for (int i = 0; i < E; ++i) e[i] = ex2(exponent(Elem<T>::get(q[j], i)));
 #pragma unroll
-          for (int w = E / 2; w > 0; w >>= 1)
+            for (int w = E / 2; w > 0; w >>= 1)
 #pragma unroll
-            for (int i = 0; i < w; ++i) e[i] += e[i + w];
-          z[j] = e[0];
-        }
+              for (int i = 0; i < w; ++i) e[i] += e[i + w];
+            z[j] = e[0];
+          }
+        };
+        if (sum.c == sum.c) terms([&](float v) { return fmaf(v, kL2e, -sum.c); });
+        else terms([&](float v) { return __fmul_rn(__fsub_rn(v, sum.ref), kL2e); });
         if ((z[0] + z[1]) + (z[2] + z[3]) < 1e30f) {
           sum.S += (widen_pos(z[0]) + widen_pos(z[1])) + (widen_pos(z[2]) + widen_pos(z[3]));
         } else if (sum.ref > -INFINITY) {  // (nothing but -inf so far: nothing to add)
-          sum.S = lp_tile_slow<T>(sum.S, sum.ref, p.body, t * kLpChunks * kLpThreads + tid, nchunk);  // (a NaN, an infinity, or a reference far from zero)
+          sum.S = lp_tile_slow<T>(sum.S, sum.ref, p.body, t * kLpChunks * kLpThreads + tid, nchunk);  // (a NaN or an infinity)
         }
       }
       // ---- a tile that may hold one of the n best is noted, to be looked into at the piece's end
       if (TOP && t > 0) {
-        const uint32_t nk = sm_ld_volatile(&sh.nkey);
-        uint32_t at = 0u;
-        if (tm >= floor_value(nk)) {
-          at = sm_atomic_add(&sh.rec, 1u);
-          if (at < (uint32_t)kLpRec<TOP>) {
-            sh.rec_max[at] = tm;
-            sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
+        const bool hot = tm >= floor_value(sm_ld_volatile(&sh.nkey));
+        if (__any_sync(0xFFFFFFFFu, hot)) {
+          uint32_t at = 0u;
+          if (hot) {
+            at = sm_atomic_add(&sh.rec, 1u);
+            if (at < (uint32_t)kLpRec<TOP>) {
+              sh.rec_max[at] = tm;
+              sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
+            }
+          }
+          if (__any_sync(0xFFFFFFFFu, at >= mark && at < (uint32_t)kLpRec<TOP>)) {
+            mark = __reduce_max_sync(0xFFFFFFFFu, at) + kLpMark<TOP>;
+            publish();
+            __syncwarp();
+            lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
           }
         }
-        const bool many = __any_sync(0xFFFFFFFFu, at >= mark && at < (uint32_t)kLpRec<TOP>);
-        if (t == point || many) {
+        if (t == point) {
           // (no barrier: what another warp has not published yet only leaves the threshold lower.
-          //  The warps take turns at raising it, but for one that finds many notes.)
+          //  The warps take turns at raising it.)
           publish();
           __syncwarp();
-          if (many || (tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
-          if (many) mark = __reduce_max_sync(0xFFFFFFFFu, at) + kLpMark<TOP>;
-          if (t == point) point = 2 * point + 1;
+          if ((tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
+          point = 2 * point + 1;
         }
       }
     };
@@ -689,7 +699,8 @@ static bool lp_whole(int32_t B, int32_t V) { return B >= kLpManyRows || V <= kLp
 // once: a row is cut only where one CTA's share ends. A row's units lie with at most max_pieces CTAs.
 // Where that would be less than kLpOwnPiece columns a CTA, no CTA gets the end of one row and the
 // beginning of the next, which would cost it a second piece's fixed time (7 us with alternatives: 56 x
-// 30000 fp32, 5 alternatives, 20 us when runs straddle rows, 15 before): a unit to a CTA.
+// 30000 fp32, 5 alternatives, 20 us when runs straddle rows, 15 when not): a unit to a CTA. Up to twice
+// as many columns, too, where that leaves an eighth of the CTAs without a unit at most.
 constexpr int32_t kLpOwnPiece = 8192;
 struct LpPlan {
   int32_t unit, row_units, max_pieces;
@@ -707,8 +718,10 @@ static LpPlan lp_plan(int32_t B, int32_t V, int32_t top_n) {
     return p;
   }
   const int32_t ctas = kSmCount * lp_per_sm(top_n > 0);
-  const int32_t most = (int64_t)B * V < (int64_t)ctas * kLpOwnPiece ? std::min(kMaxSeg, std::max(1, ctas / B)) : kMaxSeg;
-  p.unit = std::max(2048, ((V - 1) / most + 2048) / 2048 * 2048);
+  const int64_t share = (int64_t)B * V / ctas;
+  const bool own = share < kLpOwnPiece || (share < 2 * kLpOwnPiece && ctas / B * B * 8 >= ctas * 7);
+  const int32_t most = own ? std::min(kMaxSeg, std::max(1, ctas / B)) : kMaxSeg;
+  p.unit = std::max(top_n > 0 ? 4096 : 2048, ((V - 1) / most + 2048) / 2048 * 2048);  // (a list costs more to merge than a sum)
   p.row_units = (V + p.unit - 1) / p.unit;
   const uint32_t total = (uint32_t)B * (uint32_t)p.row_units;
   p.grid = std::min<uint32_t>(total, (uint32_t)ctas);

@@ -48,25 +48,6 @@ struct ResShared {
 // the columns, the adjusted columns (key, id)
 __host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)(max_hist + 4) * 8 + (size_t)max_bias * 8 + (size_t)(max_hist + max_bias) * 12; }
 
-__device__ __forceinline__ uint32_t cluster_addr(const void* p, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_addr(p)), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_ld(const void* p, uint32_t rank) {
-  uint32_t v;
-  asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(cluster_addr(p, rank)) : "memory");
-  return v;
-}
-__device__ __forceinline__ unsigned long long cluster_ld64(const void* p, uint32_t rank) {
-  unsigned long long v;
-  asm volatile("ld.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(cluster_addr(p, rank)) : "memory");
-  return v;
-}
-// (not the aligned forms: these stand behind code that a warp's lanes leave at different times)
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
-
 template <typename T>
 __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_constant__ SampleDev a, int ctas, int slice) {
   extern __shared__ __align__(128) char res_smem[];
