@@ -40,13 +40,33 @@ struct ResShared {
   int32_t ti[kTmpCap];
   float sv[ARCS_KCAP];
   int32_t sid[ARCS_KCAP];
-  int cnt, mcnt, misc[8], n_hist, n_touch, failed, off[17];
+  int cnt, mcnt, misc[8], n_touch, failed, off[17];
   uint32_t scal[16];                        // the elements before and after the aligned body, as float bits
 };
 
-// history entries of the slice (column, place: padded to four), the row's bias list, what applies to
-// the columns, the adjusted columns (key, id)
-__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)(max_hist + 4) * 8 + (size_t)max_bias * 8 + (size_t)(max_hist + max_bias) * 12; }
+// Slots of the table of a slice's history columns: at most three quarters of them are taken.
+__host__ __device__ inline int res_slots(int max_hist) {
+  if (max_hist <= 0) return 0;
+  int slots = 32;
+  while (3 * slots < 4 * max_hist) slots <<= 1;
+  return slots;
+}
+// the table (column, what is known of it), the row's bias list (id, value, what applies), the adjusted
+// columns (key, id)
+__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)res_slots(max_hist) * 8 + (size_t)max_bias * 12 + (size_t)(max_hist + max_bias) * 8; }
+
+// the place of a column in the table (linear probing; -1: not there), entered first if `enter`
+__device__ __forceinline__ int res_find(int32_t* h_col, int slots, int32_t c, bool enter) {
+  if (slots == 0) return -1;
+  uint32_t at = ((uint32_t)c * 2654435761u >> 12) & (uint32_t)(slots - 1);
+  for (int n = 0; n < slots; ++n) {
+    const int32_t was = enter ? (int32_t)sm_atomic_cas(&h_col[at], 0xFFFFFFFFu, (uint32_t)c) : h_col[at];
+    if (was == c) return (int)at;
+    if (was == -1) return enter ? (int)at : -1;
+    at = (at + 1) & (uint32_t)(slots - 1);
+  }
+  return -1;  // (not reached when entering: the table has more places than the history has entries)
+}
 
 template <typename T>
 __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_constant__ SampleDev a, int ctas, int slice) {
@@ -54,12 +74,13 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   ResShared& s = *reinterpret_cast<ResShared*>(res_smem);
   constexpr int E = Elem<T>::kPerChunk;
   constexpr int NT = kResThreads;
+  const int all_slots = res_slots(a.max_hist);
   int32_t* const h_col = reinterpret_cast<int32_t*>(res_smem + ((sizeof(ResShared) + 15) & ~(size_t)15));
-  int32_t* const h_at = h_col + a.max_hist + 4;
-  int32_t* const b_id = h_at + a.max_hist + 4;
+  uint32_t* const h_info = reinterpret_cast<uint32_t*>(h_col + all_slots);
+  int32_t* const b_id = reinterpret_cast<int32_t*>(h_info + all_slots);
   float* const b_val = reinterpret_cast<float*>(b_id + a.max_bias);
-  uint32_t* const info = reinterpret_cast<uint32_t*>(b_val + a.max_bias);
-  uint32_t* const t_key = info + a.max_hist + a.max_bias;
+  uint32_t* const b_info = reinterpret_cast<uint32_t*>(b_val + a.max_bias);
+  uint32_t* const t_key = b_info + a.max_bias;
   int32_t* const t_id = reinterpret_cast<int32_t*>(t_key + a.max_hist + a.max_bias);
   char* const data = res_smem + (((size_t)(reinterpret_cast<char*>(t_id + a.max_hist + a.max_bias) - res_smem) + 127) & ~(size_t)127);
 
@@ -80,7 +101,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       mbar_expect_tx(&s.bars[i], (uint32_t)n * 16u);
       bulk_load(data + (size_t)i * part * 16, p.body + (size_t)i * part * 16, (uint32_t)n * 16u, &s.bars[i]);
     }
-    s.cnt = s.n_hist = s.n_touch = s.failed = 0;
+    s.cnt = s.n_touch = s.failed = 0;
   }
   const RowCfg r = row_cfg<false>(a, b);
   if (rank == 0 && tid == 0) {
@@ -91,22 +112,39 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   const int sc_n = p.head_n + p.tail_n;
   const int32_t sc_col = tid < p.head_n ? lo + tid : p.tail_first + tid - p.head_n;
   if (tid < sc_n) s.scal[tid] = __float_as_uint(Elem<T>::load(row + sc_col));
-  __syncthreads();
-
   // ---- the listed columns of the slice
   const bool lists = r.touched_on;
   const int L_all = lists && r.pen_on ? r.H : 0, NB = lists ? r.NB : 0;
+  const int slots = res_slots(L_all);  // (what this row's history takes of the table)
+  for (int i = tid; i < slots; i += NT) {
+    h_col[i] = -1;
+    h_info[i] = 0u;
+  }
+  __syncthreads();
   if (lists) {
     const int32_t Vg = a.v_global > 0 ? a.v_global : a.V;
-    for (int i0 = 0; i0 < L_all; i0 += NT) {
-      const int i = i0 + tid;
-      const int32_t t = i < L_all ? __ldg(&a.hist_ids[r.h0 + i]) : -1;
-      const int32_t c = t >= 0 && t < Vg ? t - a.id_base : -1;
-      if (c >= lo && c < hi) {
-        const int at = (int)sm_atomic_add(&s.n_hist, 1u);
-        h_col[at] = c;
-        h_at[at] = i;
+    const int32_t w0 = window_start(r);
+    // A column of the table counts its occurrences in the history and holds whether one lies in the
+    // repeat window (bit 31). A warp enters a column it holds several times once.
+    constexpr int kAhead = 4;  // entries a thread fetches at once
+    for (int i0 = 0; i0 < L_all; i0 += kAhead * NT) {
+      int32_t t[kAhead];
+#pragma unroll
+      for (int x = 0; x < kAhead; ++x) t[x] = i0 + x * NT + tid < L_all ? __ldg(&a.hist_ids[r.h0 + i0 + x * NT + tid]) : -1;
+#pragma unroll
+      for (int x = 0; x < kAhead; ++x) {
+        const int32_t c = t[x] >= 0 && t[x] < Vg ? t[x] - a.id_base : -1;
+        const bool in = c >= lo && c < hi;
+        const unsigned any = __ballot_sync(0xFFFFFFFFu, in);
+        if (!in) continue;
+        const unsigned same = __match_any_sync(any, c);
+        if (lane != __ffs(same) - 1) continue;
+        const int at = res_find(h_col, slots, c, true);
+        const int last = i0 + x * NT + (tid & ~31) + 31 - __clz(same);
+        sm_red_add(&h_info[at], (uint32_t)__popc(same));
+        if (last >= w0) sm_red_or(&h_info[at], 1u << 31);
       }
+      __syncwarp();
     }
     for (int i = tid; i < NB; i += NT) {
       b_id[i] = __ldg(&a.bias_ids[r.q0 + i]);
@@ -119,50 +157,28 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
     if (i * part < nchunk) ok = ok && mbar_wait_warp(&s.bars[i], 0u);
   };
   if (lists) {
-    const int L = s.n_hist;
-    const int32_t w0 = window_start(r);
-    if (tid < 4) h_col[L + tid] = -1;
-    __syncthreads();
-    // What applies to a column, while the slice is on its way: its occurrences in the history, whether
-    // one lies in the repeat window (bit 31), and whether the entry at place `at` is its first (else 0).
-    auto occurrences = [&](int32_t c, int32_t at, bool& first) -> uint32_t {
-      uint32_t cnt = 0, win = 0;
-#pragma unroll 4
-      for (int j = 0; j < L; j += 4) {
-        const int4 q = *reinterpret_cast<const int4*>(&h_col[j]);
-        if (q.x == c || q.y == c || q.z == c || q.w == c) {
-          const int32_t e[4] = {q.x, q.y, q.z, q.w};
-#pragma unroll
-          for (int x = 0; x < 4; ++x)
-            if (e[x] == c) {
-              ++cnt;
-              if (h_at[j + x] >= w0) win = 1u << 31;
-              first = first && h_at[j + x] >= at;
-            }
-        }
-      }
-      return cnt | win;
-    };
-    // (a column is taken by its first bias entry, or, without one, by its first history entry)
+    // What applies to a column, while the slice is on its way. It is taken by its first bias entry, or,
+    // without one, by its place in the table.
     constexpr uint32_t kTake = 1u << 30;
     for (int i = tid; i < NB; i += NT) {
       const int32_t c = b_id[i] - a.id_base;
-      bool first = b_id[i] >= 0 && c >= lo && c < hi, none = true;
+      bool first = b_id[i] >= 0 && c >= lo && c < hi;
       for (int j = 0; j < i && first; ++j) first = b_id[j] != b_id[i];
-      info[i] = first ? kTake | occurrences(c, -1, none) : 0u;
+      const int at = first ? res_find(h_col, slots, c, false) : -1;
+      b_info[i] = first ? kTake | (at >= 0 ? h_info[at] : 0u) : 0u;
     }
-    for (int i = tid; i < L; i += NT) {
+    __syncthreads();
+    for (int i = tid; i < slots; i += NT) {
       const int32_t c = h_col[i];
-      bool first = true;
+      bool first = c >= 0;
       for (int j = 0; j < NB && first; ++j) first = b_id[j] != c + a.id_base;
-      const uint32_t o = first ? occurrences(c, h_at[i], first) : 0u;
-      info[NB + i] = first ? kTake | o : 0u;
+      if (first) h_info[i] |= kTake;
     }
     __syncthreads();
     for (int i = 0; i < kResParts; ++i) wait_part(i);
     // one column adjusted (tools/sampler.h:154-174): the raw logit from the slice, a NaN into its place
-    for (int i = tid; i < NB + L; i += NT) {
-      const uint32_t o = info[i];
+    for (int i = tid; i < NB + slots; i += NT) {
+      const uint32_t o = i < NB ? b_info[i] : h_info[i - NB];
       if (!(o & kTake)) continue;
       const int32_t c = i < NB ? b_id[i] - a.id_base : h_col[i - NB];
       float v;

@@ -100,6 +100,31 @@ def test_where_the_route_changes(V, B):
     check_rows(out, x, False, params, hists, us, rows=range(0, B, max(1, B // 12)))
 
 
+@pytest.mark.parametrize("H", [1, 31, 33, 257, 1100, 2000])
+def test_histories_that_repeat(H):
+    """one id throughout, few ids, ids as text repeats them, low ids only; windows that begin inside;
+    biases on ids of the history and on others"""
+    from arcinfer_b200 import capi
+    from gpuutil import check_rows, run_gpu_sample
+
+    g = np.random.default_rng(H)
+    V, B = 30011, 8
+    assert all(capi.lib.arcs_sample_launches(B, V, t, 0, H, 4) == 1 for t in (0, 1))
+    x = (g.standard_normal((B, V), dtype=np.float32) * 2).astype(np.float32)
+    kinds = [np.full(H, 17), g.integers(0, 3, H), np.minimum(g.zipf(1.3, H), V) - 1, g.integers(0, 300, H), g.integers(0, V, H), np.arange(H) % 40, np.full(H, V - 1), g.integers(-2, V + 3, H)]
+    hists = [k.astype(np.int32) for k in kinds]
+    x[:, :40] += 8.0  # what repeats is likely
+    params = synth.make_params(B, top_k=40, top_p=0.95, repeat_penalty=1.15, presence_penalty=0.2, frequency_penalty=0.01)
+    params["repeat_last_n"] = [-1, 64, 10, 256, 0, 5, 64, -1]
+    biases = [[(17, 1.5), (int(h[0]), -0.5), (int(h[-1]), -100.0 if b % 4 == 3 else 2.0), (V - 2, 3.0)] for b, h in enumerate(hists)]
+    us = g.random(B)
+    for bf16 in (False, True):
+        xb = synth.f32_to_bf16_bits(x) if bf16 else x
+        for bias in (None, biases):
+            out = run_gpu_sample(xb, bf16, params, hists, us, bias)
+            check_rows(out, xb, bf16, params, hists, us, bias)
+
+
 def test_long_lists_take_the_other_route():
     from gpuutil import check_rows, run_gpu_sample
 
