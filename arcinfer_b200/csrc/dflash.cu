@@ -117,10 +117,11 @@ __global__ void __launch_bounds__(32) dflash_path_kernel(const DflDev a) {
 }
 
 constexpr int kDflThreads = 256;
-constexpr int kDflMaxSteps = 8;
+constexpr int kDflMaxSteps = 8;  // most positions, and candidates, for which all pairs are scored first
+constexpr int kDflScoreK = 16;
 // words of a codebook row in shared memory: odd, so that a column's K entries lie in different banks
-__host__ __device__ inline int dfl_row_words(int rank) { return ((rank + 1) / 2) | 1; }
-static size_t dfl_score_smem(int K, int rank) { return (size_t)K * K * 8 + (size_t)K * (rank + 1) * 4 + (size_t)K * dfl_row_words(rank) * 4; }
+__host__ __device__ constexpr int dfl_row_words(int rank) { return ((rank + 1) / 2) | 1; }
+static constexpr size_t dfl_score_smem(int K, int rank) { return (size_t)K * K * 8 + (size_t)K * (rank + 1) * 4 + (size_t)K * dfl_row_words(rank) * 4; }
 
 // One CTA per position and slot: every candidate's score after every candidate of the position
 // before (after the slot's token at the first position), a pair to a thread, and the winner for
@@ -185,8 +186,8 @@ __global__ void __launch_bounds__(kDflThreads) dflash_score_kernel(const DflDev 
 // The walk over the winners: one warp per slot; all it may need is fetched at once.
 template <typename T>
 __global__ void __launch_bounds__(32) dflash_walk_kernel(const DflDev a) {
-  __shared__ int32_t win[kDflMaxSteps * kDflMaxK], id[kDflMaxSteps * kDflMaxK];
-  __shared__ float lg[kDflMaxSteps * kDflMaxK];
+  __shared__ int32_t win[kDflMaxSteps * kDflScoreK], id[kDflMaxSteps * kDflScoreK];
+  __shared__ float lg[kDflMaxSteps * kDflScoreK];
   __shared__ double lse[kDflMaxSteps];
   const int s = blockIdx.x, lane = threadIdx.x, K = a.K;
   const size_t row0 = (size_t)s * a.nd;
@@ -295,14 +296,18 @@ extern "C" int arcs_dflash_select(const arcs_dflash_args* g, void* stream) {
   a.path_p = g->path_p;
   a.status = g->status;
   a.win = reinterpret_cast<int32_t*>(p + lp_bytes + up256(R * K * 4) + up256(R * K * 8) + up256(R * 8));
-  // All pairs scored first while that is little work for the whole GPU: with the walk a call
-  // of 8 slots x 7 positions, K 16, rank 256 goes 78 -> 62 us, a warp per slot scoring as it goes -> this
-  const size_t smem = dfl_score_smem(K, a.rank);
-  if (a.steps >= 1 && a.steps <= kDflMaxSteps && smem <= 160 * 1024 && (double)g->slots * a.steps * K * K * a.rank <= 64e6) {
+  // All pairs scored first, or scored as the path is walked? The one takes K * K / 256 chains of `rank`
+  // additions whatever the positions, and fills the GPU; the other one chain a position (two above K
+  // 32). Measured in us, all pairs / walk (V 20000, with the pass over the logits): rank 256, K 16, 7
+  // positions: 1 slot 38 / 55, 64 slots 62 / 68, 150 slots 93 / 87; 2 positions 37 / 31. K 8: 7
+  // positions 32 / 52, 150 slots 71 / 84, 2 positions 31 / 30. K 32: 64 / 63, 64 slots 99 / 74. K 64:
+  // 141 / 101. Ranks 64 and 1024 fall alike (K 16, 7 positions: 32 / 38 and 68 / 130).
+  if (K <= kDflScoreK && a.steps >= (K > 8 ? 4 : 3) && a.steps <= kDflMaxSteps && (int64_t)g->slots * a.steps * K * K <= 1024 * kSmCount) {
+    const size_t smem = dfl_score_smem(K, a.rank);
 #define ARCS_LAUNCH(T)                                                                                        \
   do {                                                                                                        \
     static std::atomic<unsigned long long> attr_done{0};                                                      \
-    const cudaError_t e = ensure_dynamic_smem(dflash_score_kernel<T>, 160 * 1024, attr_done);                 \
+    const cudaError_t e = ensure_dynamic_smem(dflash_score_kernel<T>, (int)dfl_score_smem(kDflScoreK, kDflMaxRank), attr_done); \
     if (e != cudaSuccess) return set_error(ARCS_ERR_CUDA, cudaGetErrorString(e));                             \
     dflash_score_kernel<T><<<(unsigned)(g->slots * a.steps), kDflThreads, smem, st>>>(a);                     \
     dflash_walk_kernel<T><<<(unsigned)g->slots, 32, 0, st>>>(a);                                              \

@@ -11,6 +11,12 @@ from test_oracle_pin import dflash_case
 pytestmark = pytest.mark.gpu
 
 
+@pytest.mark.parametrize("V,rank,nd,topk,slots", [(700, 64, 3, 16, 2), (700, 64, 4, 16, 2), (700, 64, 4, 17, 2), (700, 64, 2, 8, 2), (700, 64, 3, 8, 2), (700, 64, 3, 9, 2),
+                                                  (700, 1024, 4, 16, 2), (500, 32, 4, 16, 148), (500, 32, 4, 16, 149)])
+def test_about_the_rule(V, rank, nd, topk, slots):
+    test_either_route(V, rank, nd, topk, slots)
+
+
 @pytest.mark.parametrize("V,rank,nd,topk,slots", [(900, 1, 7, 16, 3), (900, 7, 8, 1, 2), (900, 33, 8, 33, 3), (900, 255, 9, 16, 2), (700, 256, 1, 64, 2),
                                                   (700, 400, 7, 64, 3), (700, 1024, 3, 64, 2), (600, 256, 7, 16, 150), (600, 256, 7, 32, 40)])
 def test_either_route(V, rank, nd, topk, slots):
