@@ -157,30 +157,31 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
     if (i * part < nchunk) ok = ok && mbar_wait_warp(&s.bars[i], 0u);
   };
   if (lists) {
-    // What applies to a column, while the slice is on its way. It is taken by its first bias entry, or,
-    // without one, by its place in the table.
-    constexpr uint32_t kTake = 1u << 30;
+    // What applies to a column, while the slice is on its way. It is taken by its first bias entry (bit 30
+    // set there), or, without one, by its place in the table (bit 30 not set).
+    constexpr uint32_t kBias = 1u << 30;
     for (int i = tid; i < NB; i += NT) {
       const int32_t c = b_id[i] - a.id_base;
       bool first = b_id[i] >= 0 && c >= lo && c < hi;
       for (int j = 0; j < i && first; ++j) first = b_id[j] != b_id[i];
-      const int at = first ? res_find(h_col, slots, c, false) : -1;
-      b_info[i] = first ? kTake | (at >= 0 ? h_info[at] : 0u) : 0u;
-    }
-    __syncthreads();
-    for (int i = tid; i < slots; i += NT) {
-      const int32_t c = h_col[i];
-      bool first = c >= 0;
-      for (int j = 0; j < NB && first; ++j) first = b_id[j] != c + a.id_base;
-      if (first) h_info[i] |= kTake;
+      uint32_t o = 0u;
+      if (first) {
+        o = kBias;
+        const int at = res_find(h_col, slots, c, false);
+        if (at >= 0) {
+          o |= h_info[at];
+          h_info[at] = o;
+        }
+      }
+      b_info[i] = o;
     }
     __syncthreads();
     for (int i = 0; i < kResParts; ++i) wait_part(i);
     // one column adjusted (tools/sampler.h:154-174): the raw logit from the slice, a NaN into its place
     for (int i = tid; i < NB + slots; i += NT) {
       const uint32_t o = i < NB ? b_info[i] : h_info[i - NB];
-      if (!(o & kTake)) continue;
       const int32_t c = i < NB ? b_id[i] - a.id_base : h_col[i - NB];
+      if (i < NB ? !(o & kBias) : c < 0 || (o & kBias)) continue;
       float v;
       if (c >= p.body_first && c < p.tail_first) {
         T* at = reinterpret_cast<T*>(data) + (c - p.body_first);
@@ -198,7 +199,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
         if (b_val[j] > -100.0f) v = __fadd_rn(v, b_val[j]);
         else ban = true;
       }
-      const uint32_t cnt = o & (kTake - 1u);
+      const uint32_t cnt = o & (kBias - 1u);
       if (cnt > 0) v = penalise(r, v, cnt, (o >> 31) != 0u);
       if (ban) v = ARCS_BANNED;                                                                        // :174
       const int at = (int)sm_atomic_add(&s.n_touch, 1u);
