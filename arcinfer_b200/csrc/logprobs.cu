@@ -13,10 +13,13 @@
 //
 // What bounds it: memory, then the special-function unit (one ex2 per logit, 16 a clock and SM:
 // 59 us for 1024 x 262144, next to 83 us for its 537 MB); what the kernel takes on top are the pieces'
-// ends and beginnings. 1024 x 262144 bf16: 20 alternatives 216 -> 140 us, none 134 -> 113 us; 512 x
-// 151936 fp32, none: 80 -> 59 us (a row through a shared-memory ring with two barriers a tile, the
-// candidates' buffer kept by the whole CTA, -> this; graph replays).
+// ends and beginnings. 1024 x 262144 bf16: 20 alternatives 216 -> 147 us, none 134 -> 114 us; 512 x
+// 151936 fp32, none: 80 -> 62 us; 8 x 151936 fp32, 20 alternatives 22 -> 15 us (a row through a
+// shared-memory ring with two barriers a tile, the candidates' buffer kept by the whole CTA, -> this;
+// graph replays). A masked front of a row (7 of 8 columns, 512 x 262144 bf16, 20 alternatives): -inf
+// 410 -> 59 us, -1e30 432 -> 110.
 #include <algorithm>
+#include <type_traits>
 
 #include "plan.h"
 #include "select.cuh"
@@ -37,7 +40,7 @@ constexpr int kLpFew = 64;                    // up to so many alternatives one 
 // records a CTA keeps of threads and tiles whose maximum reached the threshold of the moment: one a thread of
 // the first tile, then about as many as alternatives wanted (plus a seventh) each time the piece doubles.
 // Each time another kLpMark have come the threshold is raised out of turn (a masked region has ended).
-template <int TOP> constexpr int kLpRec = TOP == 0 ? 1 : TOP == 1 ? 1024 : 3072;
+template <int TOP> constexpr int kLpRec = TOP == 0 ? 1 : TOP == 1 ? 1536 : 3072;
 template <int TOP> constexpr uint32_t kLpMark = TOP == 0 ? 0 : (kLpRec<TOP> - kLpThreads) / 4;
 
 struct LpPart {      // what a piece leaves for the merge
@@ -167,6 +170,29 @@ __device__ __noinline__ double lp_tile_slow(double S, float ref, const char* bod
     for (int e = 0; e < Elem<T>::kPerChunk; ++e) z += s.term(Elem<T>::get(q, e));  // (none exceeds the reference)
   }
   return S + z * exp2(s.off());
+}
+// The sums of a tile's chunks relative to a reference far from zero, the tile read once more (with
+// alternatives the loop has no registers left for a second form of the terms).
+template <typename T>
+__device__ __noinline__ float4 lp_terms_far(float ref, const char* body, int first, int nchunk) {
+  constexpr int E = Elem<T>::kPerChunk;
+  static_assert(kLpChunks == 4, "a float a chunk");
+  float z[kLpChunks];
+  uint4 q[kLpChunks];
+#pragma unroll
+  for (int j = 0; j < kLpChunks; ++j) q[j] = ldg128_stream_if(body + (size_t)(first + j * kLpThreads) * 16, first + j * kLpThreads < nchunk, LpElem<T>::kNothing);
+#pragma unroll
+  for (int j = 0; j < kLpChunks; ++j) {
+    float e[E];
+#pragma unroll
+    for (int i = 0; i < E; ++i) e[i] = ex2(__fmul_rn(__fsub_rn(Elem<T>::get(q[j], i), ref), kL2e));
+#pragma unroll
+    for (int w = E / 2; w > 0; w >>= 1)
+#pragma unroll
+      for (int i = 0; i < w; ++i) e[i] += e[i + w];
+    z[j] = e[0];
+  }
+  return make_float4(z[0], z[1], z[2], z[3]);
 }
 // What the threads have published of their own maxima belongs to disjoint sets of elements, so the
 // n-th largest of it is a lower bound of the n-th largest element: the threshold (a key,
@@ -568,9 +594,9 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
     }
 
     const int tiles = (nchunk + kLpChunks * kLpThreads - 1) / (kLpChunks * kLpThreads);
-    int point = 1;  // the next tile after which the threads publish their maxima: 1, 3, 7, 15, ...
     uint32_t mark = kLpThreads + kLpMark<TOP>;  // the number of notes at which the warp does so out of turn
-    auto tile = [&](int t, const uint4 (&q)[kLpChunks], uint4 (&nq)[kLpChunks]) {
+    auto tile = [&](auto odd, int t, const uint4 (&q)[kLpChunks], uint4 (&nq)[kLpChunks]) {
+      constexpr bool kOdd = decltype(odd)::value;  // (t is odd: what only even or only odd tiles do is left out of the other's code)
       if (t + 1 < tiles) fetch(nq, t + 1);
       if (tid == 0 && t + kLpAhead < tiles) prefetch_l2(p.body + (size_t)(t + kLpAhead) * kLpTileBytes, min(kLpTileBytes, p.body_bytes - (t + kLpAhead) * kLpTileBytes));
       const float tm = LpElem<T>::tile_max(q);
@@ -580,7 +606,7 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
       } else if (TOP == 1) {
         own[0] = fmaxf(own[0], tm);
       }
-      if (t == 0) {
+      if (!kOdd && t == 0) {
         // The CTA's largest element so far is every thread's first reference: a thread then meets a
         // larger one, and pays for the rescaling of its sum, some 32 times a row and not at every
         // maximum of its own.
@@ -628,7 +654,14 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
           }
         };
         if (sum.c == sum.c) terms([&](float v) { return fmaf(v, kL2e, -sum.c); });
-        else terms([&](float v) { return __fmul_rn(__fsub_rn(v, sum.ref), kL2e); });
+        else if (TOP == 0) terms([&](float v) { return __fmul_rn(__fsub_rn(v, sum.ref), kL2e); });
+        else if (sum.ref > -INFINITY) {
+          const float4 far = lp_terms_far<T>(sum.ref, p.body, t * kLpChunks * kLpThreads + tid, nchunk);
+          z[0] = far.x;
+          z[1] = far.y;
+          z[2] = far.z;
+          z[3] = far.w;
+        } else z[0] = z[1] = z[2] = z[3] = INFINITY;
         if ((z[0] + z[1]) + (z[2] + z[3]) < 1e30f) {
           sum.S += (widen_pos(z[0]) + widen_pos(z[1])) + (widen_pos(z[2]) + widen_pos(z[3]));
         } else if (sum.ref > -INFINITY) {  // (nothing but -inf so far: nothing to add)
@@ -636,31 +669,27 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
         }
       }
       // ---- a tile that may hold one of the n best is noted, to be looked into at the piece's end
-      if (TOP && t > 0) {
-        const bool hot = tm >= floor_value(sm_ld_volatile(&sh.nkey));
-        if (__any_sync(0xFFFFFFFFu, hot)) {
-          uint32_t at = 0u;
-          if (hot) {
-            at = sm_atomic_add(&sh.rec, 1u);
-            if (at < (uint32_t)kLpRec<TOP>) {
-              sh.rec_max[at] = tm;
-              sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
-            }
-          }
-          if (__any_sync(0xFFFFFFFFu, at >= mark && at < (uint32_t)kLpRec<TOP>)) {
-            mark = __reduce_max_sync(0xFFFFFFFFu, at) + kLpMark<TOP>;
-            publish();
-            __syncwarp();
-            lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
+      if (TOP && (kOdd || t > 0)) {
+        if (tm >= floor_value(sm_ld_volatile(&sh.nkey))) {
+          const uint32_t at = sm_atomic_add(&sh.rec, 1u);
+          if (at < (uint32_t)kLpRec<TOP>) {
+            sh.rec_max[at] = tm;
+            sh.rec_at[at] = (uint32_t)t << 8 | (uint32_t)tid;
           }
         }
-        if (t == point) {
-          // (no barrier: what another warp has not published yet only leaves the threshold lower.
-          //  The warps take turns at raising it.)
+      }
+      // ---- after tiles 1, 3, 7, 15, ..., and where notes come thick (a look every four tiles: one every two
+      // costs 2 % of the kernel), the threads publish their maxima. (No barrier: what another warp has not
+      // published yet only leaves the threshold lower. The warps take turns at raising it, but each does
+      // that finds many notes.)
+      if (TOP && kOdd && (t == 1 || (t & 2) != 0)) {
+        const uint32_t rec = __shfl_sync(0xFFFFFFFFu, sm_ld_volatile(&sh.rec), 0);
+        const bool many = rec >= mark && rec < (uint32_t)kLpRec<TOP>;
+        if ((t & (t + 1)) == 0 || many) {
           publish();
           __syncwarp();
-          if ((tid >> 5) == (__ffs(point + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
-          point = 2 * point + 1;
+          if (many || (tid >> 5) == (__ffs(t + 1) & (kLpThreads / 32 - 1))) lp_raise_threshold<OWN * kLpThreads / 32>(sh.keys, n, &sh.nkey);
+          if (many) mark = rec + kLpMark<TOP>;
         }
       }
     };
@@ -670,8 +699,8 @@ __global__ void __launch_bounds__(kLpThreads, lp_per_sm(TOP != 0)) logprob_kerne
       if (bytes > 0) prefetch_l2(reinterpret_cast<const void*>(next), bytes);
     }
     for (int t = 0; t < tiles; t += 2) {
-      tile(t, qa, qb);
-      if (t + 1 < tiles) tile(t + 1, qb, qa);
+      tile(std::false_type(), t, qa, qb);
+      if (t + 1 < tiles) tile(std::true_type(), t + 1, qb, qa);
     }
     if (hv) sum.one(vh);
     if (tv) sum.one(vt);
