@@ -1,8 +1,9 @@
 // sample_batch: penalties + temperature / top-k / top-p / min-p (+ allowed-token mask) with one
-// pass over the logits. Rows that fit on the chip: one launch (sample_resident.cuh). Others: two launches on the caller's stream: stream (the pass itself, which also
-// prepares each item's touched tokens ahead of the pass) and finish (per row: order, softmax,
-// cuts, draw), which runs beside the stream kernel and takes each row as it is released. The
-// kernels hand their results on through the workspace.
+// pass over the logits. Rows that fit on the chip: one launch (sample_resident.cuh). Others: two
+// launches on the caller's stream: stream (the pass itself, which also prepares each item's touched
+// tokens ahead of the pass) and finish (per row: order, softmax, cuts, draw), which runs beside the
+// stream kernel and takes each row as it is released. The kernels hand their results on through the
+// workspace.
 #include <algorithm>
 
 #include "sample_finish.cuh"

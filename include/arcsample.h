@@ -357,7 +357,8 @@ int arcs_logprobs_batch(const arcs_logprob_args* args, void* stream);
  * log-sum-exp (logprobs_batch), within 1e-7 relative of the exact sum where the reference's
  * float sums over blocks of 4096 are within about 1e-6: a path probability that close to min_p
  * may be cut one draft apart.
- * The first step is arcs_logprobs_batch on slots * nd rows; the second one warp per slot.
+ * The first step is arcs_logprobs_batch on slots * nd rows; the second walks a slot's path, scoring as
+ * it goes or over winners found for all pairs of candidates beforehand.
  * ---------------------------------------------------------------------------------------- */
 typedef struct {
   const void* logits;      /* [slots][nd][row_stride] device, of dtype */

@@ -73,7 +73,8 @@ def test_many_rows_one_segment():
 @pytest.mark.parametrize("masked", [False, True])
 def test_ascending_rows_overflow_the_lists(masked):
     """ascending logits make every element a survivor of the stream: the per-item lists overflow
-    and the rows are read again by the finishing step; same results as ever"""
+    and the rows are read again by the finishing step; same results as ever (without a mask these few
+    rows are held on the chip: the streaming route has them in test_gpu_stream_route.py)"""
     from gpuutil import check_rows, run_gpu_sample
 
     g = np.random.default_rng(310 + masked)
