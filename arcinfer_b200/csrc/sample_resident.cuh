@@ -3,10 +3,10 @@
 // While the rows of a call fit on the chip, a cluster of CTAs takes each: every CTA fetches one slice
 // of the row with bulk copies (TMA) and keeps it, so that nothing has to be handed from one kernel
 // to another, and no threshold has to be found before the data have passed:
-//  1. while the slice is on its way, the CTA picks the listed ids that fall into it out of the row's
-//     history and bias lists;
+//  1. while the slice is on its way, the CTA enters the history's ids that fall into it in a hash
+//     table, which counts them, and looks the biases' columns up there;
 //  2. each such column is adjusted with the exact fp32 arithmetic of Sampler::adjusted
-//     (tools/sampler.h:147-176) and goes to a list of its own; a NaN takes its place in the slice;
+//     (tools/sampler.h:147-176) and kept in the table; a NaN takes its place in the slice;
 //  3. the k-th largest of the threads' own maxima bounds the slice's k-th element from below; what
 //     reaches it, and the adjusted columns that do, are the slice's candidates (a few more than k);
 //  4. the cluster's first CTA reads the others' candidates out of their shared memory, ranks them
@@ -40,20 +40,19 @@ struct ResShared {
   int32_t ti[kTmpCap];
   float sv[ARCS_KCAP];
   int32_t sid[ARCS_KCAP];
-  int cnt, mcnt, misc[8], n_touch, failed, off[17];
+  int cnt, mcnt, misc[8], failed, off[17];
   uint32_t scal[16];                        // the elements before and after the aligned body, as float bits
 };
 
-// Slots of the table of a slice's history columns: at most three quarters of them are taken.
+// Slots of the table of a slice's history columns: at most four fifths of them are taken.
 __host__ __device__ inline int res_slots(int max_hist) {
   if (max_hist <= 0) return 0;
-  int slots = 32;
-  while (3 * slots < 4 * max_hist) slots <<= 1;
+  int slots = 2;
+  while (4 * slots < 5 * max_hist) slots <<= 1;
   return slots;
 }
-// the table (column, what is known of it), the row's bias list (id, value, what applies), the adjusted
-// columns (key, id)
-__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)res_slots(max_hist) * 8 + (size_t)max_bias * 12 + (size_t)(max_hist + max_bias) * 8; }
+// the table (column, what is known of it and then its adjusted key), the row's bias list (id, value, the same)
+__host__ __device__ inline size_t res_list_bytes(int max_hist, int max_bias) { return (size_t)res_slots(max_hist) * 8 + (size_t)max_bias * 12; }
 
 // the place of a column in the table (linear probing; -1: not there), entered first if `enter`
 __device__ __forceinline__ int res_find(int32_t* h_col, int slots, int32_t c, bool enter) {
@@ -80,9 +79,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   int32_t* const b_id = reinterpret_cast<int32_t*>(h_info + all_slots);
   float* const b_val = reinterpret_cast<float*>(b_id + a.max_bias);
   uint32_t* const b_info = reinterpret_cast<uint32_t*>(b_val + a.max_bias);
-  uint32_t* const t_key = b_info + a.max_bias;
-  int32_t* const t_id = reinterpret_cast<int32_t*>(t_key + a.max_hist + a.max_bias);
-  char* const data = res_smem + (((size_t)(reinterpret_cast<char*>(t_id + a.max_hist + a.max_bias) - res_smem) + 127) & ~(size_t)127);
+  char* const data = res_smem + (((size_t)(reinterpret_cast<char*>(b_info + a.max_bias) - res_smem) + 127) & ~(size_t)127);
 
   const int tid = threadIdx.x, lane = tid & 31;
   const int rank = (int)blockIdx.x % ctas, b = (int)blockIdx.x / ctas;
@@ -101,7 +98,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       mbar_expect_tx(&s.bars[i], (uint32_t)n * 16u);
       bulk_load(data + (size_t)i * part * 16, p.body + (size_t)i * part * 16, (uint32_t)n * 16u, &s.bars[i]);
     }
-    s.cnt = s.n_touch = s.failed = 0;
+    s.cnt = s.failed = 0;
   }
   const RowCfg r = row_cfg<false>(a, b);
   if (rank == 0 && tid == 0) {
@@ -181,7 +178,11 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
     for (int i = tid; i < NB + slots; i += NT) {
       const uint32_t o = i < NB ? b_info[i] : h_info[i - NB];
       const int32_t c = i < NB ? b_id[i] - a.id_base : h_col[i - NB];
-      if (i < NB ? !(o & kBias) : c < 0 || (o & kBias)) continue;
+      uint32_t* const key = i < NB ? &b_info[i] : &h_info[i - NB];
+      if (i < NB ? !(o & kBias) : c < 0 || (o & kBias)) {
+        *key = 0u;  // (no column of its own: as a NaN, never a candidate)
+        continue;
+      }
       float v;
       if (c >= p.body_first && c < p.tail_first) {
         T* at = reinterpret_cast<T*>(data) + (c - p.body_first);
@@ -202,9 +203,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       const uint32_t cnt = o & (kBias - 1u);
       if (cnt > 0) v = penalise(r, v, cnt, (o >> 31) != 0u);
       if (ban) v = ARCS_BANNED;                                                                        // :174
-      const int at = (int)sm_atomic_add(&s.n_touch, 1u);
-      t_key[at] = key_of(v);
-      t_id[at] = c + a.id_base;
+      *key = key_of(v);
     }
     __syncthreads();
   }
@@ -251,7 +250,9 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
   }
   __syncthreads();
   // ---- its candidates
-  const int n_touch = lists ? s.n_touch : 0;
+  const int n_list = lists ? NB + slots : 0;  // places that may hold an adjusted column
+  auto listed_key = [&](int i) { return i < NB ? b_info[i] : h_info[i - NB]; };
+  auto listed_id = [&](int i) { return i < NB ? b_id[i] : h_col[i - NB] + a.id_base; };
   const unsigned long long flo = s.floor;
   {
     const uint32_t tkey = (uint32_t)((flo + 1ull) >> 32);
@@ -285,7 +286,7 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       }
     }
     if (sc >= tf) keep(key_of(sc), sc_col + a.id_base);
-    for (int i = tid; i < n_touch; i += NT) keep(t_key[i], t_id[i]);
+    for (int i = tid; i < n_list; i += NT) keep(listed_key(i), listed_id(i));
   }
   __syncthreads();
   if (s.cnt > kResCap) {
@@ -313,11 +314,11 @@ __global__ void __launch_bounds__(kResThreads, 2) resident_kernel(const __grid_c
       ky = key_of(sc);
       id = sc_col + a.id_base;
     });
-    for (int i0 = 0; i0 < n_touch; i0 += NT) {
+    for (int i0 = 0; i0 < n_list; i0 += NT) {
       const int i = i0 + tid;
-      push_all<NT>(sel, ps, i < n_touch ? 1u : 0u, [&](int, uint32_t& ky, int32_t& id) {
-        ky = t_key[i];
-        id = t_id[i];
+      push_all<NT>(sel, ps, i < n_list ? 1u : 0u, [&](int, uint32_t& ky, int32_t& id) {
+        ky = listed_key(i);
+        id = listed_id(i);
       });
     }
     __syncthreads();
